@@ -11,8 +11,8 @@ namespace ptb {
 //
 // One "job" is C[M][N] = sum over segments s of (+/-) A_s B_s for one
 // triple, where A_s is a [rows][K_s] slice of a padded amplitude/OOVO block
-// (TMA view: dims (K, rows, Q, P)) and B_s a [K_s][N] slice of a padded
-// OVVV/amplitude block (TMA view: dims (N, K, P)).  The slices are selected
+// (TMA view: dims (4, rows, K/4, Q, P)) and B_s a [K_s][N] slice of a padded
+// OVVV/amplitude block (TMA view: dims (4, K, N/4, P)).  The slices are selected
 // by the occupied indices (Q, P) resp. (P) of the triple.
 
 constexpr int GEMM_BM = 128;   // rows of a CTA tile (96 or 128, per case)
@@ -24,12 +24,21 @@ constexpr int GEMM_THREADS = (GEMM_CONSUMER_WARPS + 1) * 32;
 constexpr int MAX_SEG = 6;
 constexpr int MAX_MAPS = 24;
 
+// Fours of K in the last of a segment's K steps (GemmSeg::klast).
+inline int dmma_klast(int64_t k) {
+  return (int)(((k + 3) / 4 + GEMM_BK / 4 - 1) % (GEMM_BK / 4)) + 1;
+}
+
 struct GemmSeg {
   int16_t amap, bmap;   // indices into MapSet
   int16_t neg;          // neg != 0: subtract this product (INT8: the index
                         // of the first negated digit plane)
-  int16_t half_last;    // INT8: the last K chunk holds <= 32 bytes of K, so
+  union {
+    int16_t half_last;  // INT8: the last K chunk holds <= 32 bytes of K, so
                         // its second MMA K step (all zero) is skipped
+    int16_t klast;      // DMMA: fours of K in the last K step (1..4); the
+                        // zero columns after them are not multiplied
+  };
   int32_t a_q, a_p;     // A-view coordinates of dims 2 and 3
   int32_t b_p;          // B-view coordinate of dim 2
   int32_t ksteps;       // ceil(K_s / GEMM_BK)

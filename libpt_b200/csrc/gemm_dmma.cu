@@ -9,14 +9,20 @@
 // Pipeline: warp 8 (one elected lane) stages A and B tiles with TMA into a
 // GEMM_STAGES-deep ring of shared-memory buffers guarded by mbarriers;
 // warps 0-7 run mma.sync.m16n8k4.f64 on (BM/2) x 32 warp tiles.
-// BM is 96 or 128 rows; the host picks the one that pads M less (v = 477
-// fills 5 x 96 = 480 rows against 4 x 128 = 512).
+// BM is 96 or 128 rows.  A job's last M tile multiplies only the 16-row
+// fragments that hold rows of the job, shared out to the two warp rows of the
+// tile: each has one warp on every SM sub-partition, so a tile's DMMA time
+// follows its fragment count (v = 143: 144 rows of work, not 192).
 //
-// Shared-memory layouts (no swizzle; TMA boxes are 32 bytes wide):
-//   A stage [k/4][m][k%4]   -- four boxes of (4 k x BM rows)
-//   B stage [n/4][k][n%4]   -- thirty-two boxes of (4 n x 16 k)
+// Shared-memory layouts (no swizzle; TMA box rows are 32 bytes):
+//   A stage [k/4][m][k%4]   -- one box of (4 k) x BM rows x 4
+//   B stage [n/4][k][n%4]   -- one box of (4 n) x 16 k x 32
 // so the fragment loads of a half-warp read 16 consecutive doubles (no bank
-// conflicts) for both operands.
+// conflicts) for both operands.  The views split K (A) and N (B) in fours to
+// make that layout one copy per operand and stage: with a copy per box of 4
+// columns (36 per stage) the TMA unit's rate of copies, about one in 90
+// cycles, held a stage at 3.4 k cycles whatever its rows; 96 rows of DMMA
+// work take 3.1 k.
 //
 // Persistent: GEMM_GRID CTAs take the launch's tiles one at a time from the
 // tile queue of a device-memory work list (GemmList; common.cuh tq_*), so
@@ -43,6 +49,45 @@ constexpr int NCW = GEMM_CONSUMER_WARPS;
 template <int BM>
 constexpr uint32_t stage_bytes() {
   return (BM * BK + BK * BN) * sizeof(double);
+}
+
+// Four K columns of a warp: NF 16-row fragments of A times its 32 columns
+// of B.
+template <int NF, int MF>
+__device__ __forceinline__ void mma_k4(double (&acc)[MF][4][4],
+                                       const double *A, const double *B,
+                                       const int (&boff)[4],
+                                       unsigned long long mask) {
+  double a0[NF], a1[NF], b[4];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    a0[f] = flip_sign(A[64 * f], mask);
+    a1[f] = flip_sign(A[64 * f + 32], mask);
+  }
+#pragma unroll
+  for (int h = 0; h < 4; ++h) b[h] = B[boff[h]];
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+#pragma unroll
+    for (int h = 0; h < 4; ++h) dmma_16x8x4(acc[f][h], a0[f], a1[f], b[h]);
+}
+
+// One pipeline stage of a warp: its first nkq fours of K (all of them but in
+// a segment's last stage, whose remaining columns are zero).
+template <int NF, int MF, int BM>
+__device__ __forceinline__ void mma_stage(double (&acc)[MF][4][4],
+                                          const double *A, const double *B,
+                                          const int (&boff)[4],
+                                          unsigned long long mask, int nkq) {
+  if (nkq == BK / 4) {
+#pragma unroll
+    for (int kq = 0; kq < BK / 4; ++kq)
+      mma_k4<NF, MF>(acc, A + kq * BM * 4, B + kq * 16, boff, mask);
+  } else {
+#pragma unroll 1
+    for (int kq = 0; kq < nkq; ++kq)
+      mma_k4<NF, MF>(acc, A + kq * BM * 4, B + kq * 16, boff, mask);
+  }
 }
 
 // One CTA of GEMM_THREADS (9 warps) per SM.  With 9 warps one SM
@@ -109,14 +154,8 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
             double *dA = sA + stage * BM * BK;
             double *dB = sB + stage * BK * BN;
             const int k0 = ks * BK;
-#pragma unroll
-            for (int q = 0; q < BK / 4; ++q)
-              tma_load_4d(dA + q * BM * 4, am, &full[stage], k0 + 4 * q, m0,
-                          sg.a_q, sg.a_p);
-#pragma unroll 8
-            for (int r = 0; r < BN / 4; ++r)
-              tma_load_3d(dB + r * BK * 4, bm, &full[stage], n0 + 4 * r, k0,
-                          sg.b_p);
+            tma_load_5d(dA, am, &full[stage], 0, m0, k0 / 4, sg.a_q, sg.a_p);
+            tma_load_4d(dB, bm, &full[stage], 0, k0, n0 / 4, sg.b_p);
             ++issued;
             if (++stage == ST) {
               stage = 0;
@@ -138,14 +177,10 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
   }
 
   // ---------------- consumers ----------------
-  const int wm = (warp >> 2) * (BM / 2);   // warp tile origin in the CTA tile
-  const int wn = (warp & 3) * 32;
+  const int wn = (warp & 3) * 32;          // warp tile columns
   const int g = lane >> 2, t = lane & 3;
 
   // Per-lane fragment offsets inside one stage.
-  int aoff[MF];
-#pragma unroll
-  for (int f = 0; f < MF; ++f) aoff[f] = (wm + 16 * f + g) * 4 + t;
   int boff[4];
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
@@ -175,34 +210,34 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
       for (int h = 0; h < 4; ++h)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[f][h][e] = 0.0;
+    // the tile's 16-row fragments that hold rows of the job, shared out to
+    // the two warp rows (a full tile: MF each)
+    const int frags = min(2 * MF, (job.M - m0 + 15) >> 4);
+    const int f0 = (frags + 1) >> 1;
+    const int nf = (warp >> 2) ? frags - f0 : f0;
+    const int wm = (warp >> 2) ? 16 * f0 : 0;
+    const int aoff = (wm + g) * 4 + t;
 
     for (int s = 0; s < nseg && ok; ++s) {
       const unsigned long long mask =
           job.seg[s].neg ? 0x8000000000000000ull : 0ull;
-      const int nk = job.seg[s].ksteps;
+      const int nk = job.seg[s].ksteps, klast = job.seg[s].klast;
       for (int ks = 0; ks < nk; ++ks) {
+        const int nkq = ks + 1 < nk ? BK / 4 : klast;
         if (!mbar_wait(&full[stage], phase, err)) {
           ok = false;
           break;
         }
-        const double *A = sA + stage * BM * BK;
+        const double *A = sA + stage * BM * BK + aoff;
         const double *B = sB + stage * BK * BN;
-#pragma unroll
-        for (int kq = 0; kq < BK / 4; ++kq) {
-          double a0[MF], a1[MF], b[4];
-#pragma unroll
-          for (int f = 0; f < MF; ++f) {
-            a0[f] = flip_sign(A[kq * BM * 4 + aoff[f]], mask);
-            a1[f] = flip_sign(A[kq * BM * 4 + aoff[f] + 32], mask);
-          }
-#pragma unroll
-          for (int h = 0; h < 4; ++h) b[h] = B[kq * 16 + boff[h]];
-#pragma unroll
-          for (int f = 0; f < MF; ++f)
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-              dmma_16x8x4(acc[f][h], a0[f], a1[f], b[h]);
-        }
+        if (nf == MF)
+          mma_stage<MF, MF, BM>(acc, A, B, boff, mask, nkq);
+        else if (nf == 1)
+          mma_stage<1, MF, BM>(acc, A, B, boff, mask, nkq);
+        else if (nf == 2)
+          mma_stage<2, MF, BM>(acc, A, B, boff, mask, nkq);
+        else if (MF == 4 && nf == 3)
+          mma_stage<3, MF, BM>(acc, A, B, boff, mask, nkq);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == ST) {
@@ -219,6 +254,7 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
     const int M = job.M, N = job.N;
 #pragma unroll
     for (int f = 0; f < MF; ++f) {
+      if (f >= nf) break;
       const int r = m0 + wm + 16 * f + g;
 #pragma unroll
       for (int h = 0; h < 4; ++h) {

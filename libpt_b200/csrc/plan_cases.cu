@@ -328,6 +328,21 @@ int build_aab(libpt_plan *p, SpinCase &c) {
   return LIBPT_OK;
 }
 
+// Modelled SM cycles per 16-deep K step of the tile column that covers m
+// rows with tiles of bm rows: the kernel multiplies whole 16-row fragments
+// (64 FP64 multiply-adds per cycle: 32 cycles per row of a 128-column tile),
+// and a tile cannot run faster than its operands arrive (26 bytes per cycle
+// with 32-byte TMA box rows).  Only a last tile of 16 rows is bound by its
+// operands, so 97..112 rows go to one 128-row tile, not to 96 + 16.
+static int64_t dmma_row_cost(int64_t m, int64_t bm) {
+  int64_t cost = 0;
+  for (int64_t r = 0; r < m; r += bm) {
+    const int64_t rows = (std::min(bm, m - r) + 15) / 16 * 16;
+    cost += std::max<int64_t>(32 * rows, (rows + GEMM_BN) * GEMM_BK * 8 / 26);
+  }
+  return cost;
+}
+
 int add_cases(libpt_plan *p) {
   const int oa = p->oa, va = p->va, ob = p->ob, vb = p->vb;
   auto add = [&](int type, int flip, int o1, int v1, int o2, int v2) {
@@ -365,12 +380,13 @@ int add_cases(libpt_plan *p) {
   if (p->unrestricted) add(1, 1, ob, vb, oa, va);
   for (SpinCase &c : p->cases) {
     if (c.count == 0) continue;
-    // CTA tile rows: the choice that pads the GEMM rows (va, and vb for the
-    // mixed-spin P job) least; ties go to 128 (more CTAs)
-    auto padded = [](int64_t m, int64_t bm) { return (m + bm - 1) / bm * bm; };
-    const int64_t w128 = padded(c.va, 128) + (c.type ? padded(c.vb, 128) : 0);
-    const int64_t w96 = padded(c.va, 96) + (c.type ? padded(c.vb, 96) : 0);
-    c.bm = w96 < w128 ? 96 : 128;
+    // CTA tile rows: the least modelled time of the GEMM rows (va, and vb
+    // for the mixed-spin P job); ties go to 96 (no register spills)
+    const int64_t w128 = dmma_row_cost(c.va, 128) +
+                         (c.type ? dmma_row_cost(c.vb, 128) : 0);
+    const int64_t w96 = dmma_row_cost(c.va, 96) +
+                        (c.type ? dmma_row_cost(c.vb, 96) : 0);
+    c.bm = w128 < w96 ? 128 : 96;
     int r = c.type == 0 ? build_aaa(p, c) : build_aab(p, c);
     if (!r && p->precision == LIBPT_PREC_TF32X3) r = build_tc(p, c);
     if (r) return r;

@@ -30,9 +30,9 @@ inline int64_t npair(int64_t v) { return v * (v - 1) / 2; }
 inline int ksteps(int64_t k) { return (int)((k + GEMM_BK - 1) / GEMM_BK); }
 
 // ---- tensor-map views (plan_views.cu) ---------------------------------------
-// A-view of a padded block [P][Q][R][Kpad] with logical K: dims (K, R, Q, P),
-// box (4, bm, 1, 1); B-view of a padded block [P][K][Nld] with logical N:
-// dims (N, K, P), box (4, GEMM_BK, 1).
+// A-view of a padded block [P][Q][R][Kpad]: dims (4, R, Kpad/4, Q, P), box
+// (4, bm, GEMM_BK/4, 1, 1); B-view of a padded block [P][K][Nld] with logical
+// N: dims (4, K, N/4, P), box (4, GEMM_BK, GEMM_BN/4, 1).
 int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
           int64_t P, int bm);
 int map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld, int64_t K,

@@ -34,8 +34,11 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// A-view of a padded block [P][Q][R][Kpad] with logical K: dims (K, R, Q, P),
-// box (4, bm, 1, 1).
+// A-view of a padded block [P][Q][R][Kpad] with logical K: dims
+// (4, R, Kpad/4, Q, P), box (4, bm, GEMM_BK/4, 1, 1), which lands in shared
+// memory as [k/4][m][k%4].  K is split in fours so that one TMA copy brings
+// a whole stage's tile: a copy per 4 columns is bound by the TMA unit's rate
+// of copies, not by bytes (see gemm_dmma.cu).  The pad columns hold zeros.
 int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
           int64_t P, int bm) {
   if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
@@ -44,16 +47,16 @@ int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
     set_error("cuTensorMapEncodeTiled unavailable");
     return LIBPT_ERR_CUDA;
   }
-  const int64_t kp = pad4(K);
-  cuuint64_t dims[4] = {(cuuint64_t)std::max<int64_t>(K, 1),
-                        (cuuint64_t)std::max<int64_t>(R, 1),
+  const int64_t kp = pad4(std::max<int64_t>(K, 1));
+  cuuint64_t dims[5] = {4, (cuuint64_t)std::max<int64_t>(R, 1),
+                        (cuuint64_t)(kp / 4),
                         (cuuint64_t)std::max<int64_t>(Q, 1),
                         (cuuint64_t)std::max<int64_t>(P, 1)};
-  cuuint64_t strides[3] = {(cuuint64_t)(kp * 8), (cuuint64_t)(R * kp * 8),
+  cuuint64_t strides[4] = {(cuuint64_t)(kp * 8), 32, (cuuint64_t)(R * kp * 8),
                            (cuuint64_t)(Q * R * kp * 8)};
-  cuuint32_t box[4] = {4, (cuuint32_t)bm, 1, 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void *)p, dims,
+  cuuint32_t box[5] = {4, (cuuint32_t)bm, GEMM_BK / 4, 1, 1};
+  cuuint32_t es[5] = {1, 1, 1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, (void *)p, dims,
                    strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -64,8 +67,9 @@ int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
   return LIBPT_OK;
 }
 
-// B-view of a padded block [P][K][Nld] with logical N: dims (N, K, P),
-// box (4, GEMM_BK, 1).
+// B-view of a padded block [P][K][Nld] with logical N (a multiple of 4):
+// dims (4, K, N/4, P), box (4, GEMM_BK, GEMM_BN/4, 1), one copy per stage,
+// which lands in shared memory as [n/4][k][n%4].
 int map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld, int64_t K,
           int64_t P) {
   if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
@@ -74,13 +78,14 @@ int map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld, int64_t K,
     set_error("cuTensorMapEncodeTiled unavailable");
     return LIBPT_ERR_CUDA;
   }
-  cuuint64_t dims[3] = {(cuuint64_t)std::max<int64_t>(N, 1),
-                        (cuuint64_t)std::max<int64_t>(K, 1),
+  cuuint64_t dims[4] = {4, (cuuint64_t)std::max<int64_t>(K, 1),
+                        (cuuint64_t)std::max<int64_t>(pad4(N) / 4, 1),
                         (cuuint64_t)std::max<int64_t>(P, 1)};
-  cuuint64_t strides[2] = {(cuuint64_t)(Nld * 8), (cuuint64_t)(K * Nld * 8)};
-  cuuint32_t box[3] = {4, (cuuint32_t)GEMM_BK, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void *)p, dims,
+  cuuint64_t strides[3] = {(cuuint64_t)(Nld * 8), 32,
+                           (cuuint64_t)(K * Nld * 8)};
+  cuuint32_t box[4] = {4, (cuuint32_t)GEMM_BK, GEMM_BN / 4, 1};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void *)p, dims,
                    strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -177,6 +177,7 @@ int kernel_case(int precision, int m, int n, int k, int reps, double *rel_err,
       job.seg[s].bmap = (int16_t)(1 + s);
       job.seg[s].neg = (int16_t)s;
       job.seg[s].ksteps = (k + GEMM_BK - 1) / GEMM_BK;
+      job.seg[s].klast = (int16_t)dmma_klast(k);
     }
     publish(&maps, sizeof(maps));
     launch = [=]() { return gemm_dmma_launch(dj, dl, 1, nt, pmaps, bm, grid, err, nullptr); };
