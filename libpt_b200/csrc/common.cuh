@@ -274,14 +274,18 @@ __device__ __forceinline__ double recip_nr(double d) {
 // next tile while the current one is still being staged, and hands the
 // index to the CTA's other roles through a small ring in shared memory
 // (slot `full` barrier: the index is written; `empty` barrier: every
-// consumer has read it).  -1 ends the sequence.  Tiles of uneven cost (jobs
+// consumer has read it), together with the index of the tile's job: the
+// search of the job list is a chain of dependent global loads (up to 9 in a
+// launch of 300 jobs, 2-4 k cycles), which the producer makes while the tile
+// before is staged; made by the consumers it held every tile up.  -1 ends
+// the sequence.  Tiles of uneven cost (jobs
 // of different K, rounds mixing solves) then spread over the SMs instead of
 // being dealt round-robin in advance.  Every wait is bounded.
 constexpr int TQ_SLOTS = 4;
 
 struct TileRing {
   uint64_t full[TQ_SLOTS], empty[TQ_SLOTS];
-  int tile[TQ_SLOTS];
+  int tile[TQ_SLOTS], job[TQ_SLOTS];
 };
 
 // Thread 0, before the CTA's first barrier: `consumers` arrivals free a slot.
@@ -297,11 +301,12 @@ __device__ __forceinline__ int tq_take(GemmList *l) {
   return atomicAdd(&l->next, 1);
 }
 
-// Producer: publishes tile t (or -1) in the next slot.
+// Producer: publishes tile t (or -1) of job j in the next slot.
 __device__ __forceinline__ bool tq_put(TileRing *r, int &slot, uint32_t &ph,
-                                       int t, unsigned *err) {
+                                       int t, int j, unsigned *err) {
   if (!mbar_wait(&r->empty[slot], ph ^ 1u, err)) return false;
   r->tile[slot] = t;
+  r->job[slot] = j;
   mbar_arrive(&r->full[slot]);   // release: the index is visible after it
   if (++slot == TQ_SLOTS) {
     slot = 0;
@@ -311,11 +316,14 @@ __device__ __forceinline__ bool tq_put(TileRing *r, int &slot, uint32_t &ph,
 }
 
 // Consumer (every thread of a consuming warp calls it; lane 0 frees the
-// slot for the warp): the next tile index, -1 at the end or on a timeout.
+// slot for the warp): the next tile index, -1 at the end or on a timeout;
+// j = the index of its job.
 __device__ __forceinline__ int tq_get(TileRing *r, int &slot, uint32_t &ph,
-                                      unsigned *err, bool warp_arrives) {
+                                      int &j, unsigned *err,
+                                      bool warp_arrives) {
   if (!mbar_wait(&r->full[slot], ph, err)) return -1;
   const int t = r->tile[slot];
+  j = r->job[slot];
   if (warp_arrives) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(&r->empty[slot]);

@@ -130,13 +130,15 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
       // tiles from the launch's queue; the next one is taken while the
       // current one is staged
       int tile = tq_take(list);
+      int ji = find_entry(jobs, njobs, tile, &GemmJob::tile_begin);
       while (ok) {
-        if (!tq_put(tq, qslot, qph, tile < ntiles ? tile : -1, err) ||
+        if (!tq_put(tq, qslot, qph, tile < ntiles ? tile : -1, ji, err) ||
             tile >= ntiles)
           break;
         const int next_tile = tq_take(list);
-        const GemmJob &job =
-            jobs[find_entry(jobs, njobs, tile, &GemmJob::tile_begin)];
+        const int next_ji = find_entry(jobs, njobs, next_tile,
+                                       &GemmJob::tile_begin);
+        const GemmJob &job = jobs[ji];
         const int local = tile - job.tile_begin;
         const int m0 = (local % job.mtiles) * BM;
         const int n0 = (local / job.mtiles) * BN;
@@ -164,6 +166,7 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
           }
         }
         tile = next_tile;
+        ji = next_ji;
       }
       tq_finish(list);
       // Drain: do not leave the CTA while copies issued by it are in flight.
@@ -194,10 +197,10 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
   int qslot = 0;
   uint32_t qph = 0;
   for (;;) {
-    const int tile = tq_get(tq, qslot, qph, err, true);
+    int ji;
+    const int tile = tq_get(tq, qslot, qph, ji, err, true);
     if (tile < 0) break;
-    const GemmJob &job =
-        jobs[find_entry(jobs, njobs, tile, &GemmJob::tile_begin)];
+    const GemmJob &job = jobs[ji];
     const int local = tile - job.tile_begin;
     const int m0 = (local % job.mtiles) * BM;
     const int n0 = (local / job.mtiles) * BN;

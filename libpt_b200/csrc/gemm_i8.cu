@@ -406,14 +406,17 @@ __device__ __forceinline__ void i8_body(const LaunchMaps *pm,
     // tiles from the launch's queue; the next one is taken while the
     // current one is staged
     int tile = tq_take(list);
+    int ji = find_entry(jobs, njobs, tile, &GemmJob::tile_begin);
     while (ok) {
-      if (!tq_put(tq, qslot, qph, tile < ntiles ? tile : -1, err) ||
+      if (!tq_put(tq, qslot, qph, tile < ntiles ? tile : -1, ji, err) ||
           tile >= ntiles)
         break;
       const int next_tile = tq_take(list);
+      const int next_ji = find_entry(jobs, njobs, next_tile,
+                                     &GemmJob::tile_begin);
       // job fields are copied to registers: the asm memory clobbers and
       // global stores below would otherwise force reloads
-      const GemmJob &job = jobs[find_entry(jobs, njobs, tile, &GemmJob::tile_begin)];
+      const GemmJob &job = jobs[ji];
       const int local = tile - job.tile_begin;
       const int m0 = (local % job.mtiles) * BM;
       const int n0 = (local / job.mtiles) * BN;
@@ -444,6 +447,7 @@ __device__ __forceinline__ void i8_body(const LaunchMaps *pm,
         }
       }
       tile = next_tile;
+      ji = next_ji;
     }
     tq_finish(list);
   } else if (warp == 1 && lane == 0) {
@@ -456,9 +460,10 @@ __device__ __forceinline__ void i8_body(const LaunchMaps *pm,
     int qslot = 0;
     uint32_t qph = 0;
     for (;; ++it) {
-      const int tile = tq_get(tq, qslot, qph, err, false);
+      int ji;
+      const int tile = tq_get(tq, qslot, qph, ji, err, false);
       if (tile < 0) break;
-      const GemmJob &job = jobs[find_entry(jobs, njobs, tile, &GemmJob::tile_begin)];
+      const GemmJob &job = jobs[ji];
       if (!mbar_wait(accempty, (uint32_t)((it & 1) ^ 1), err)) {
         ok = false;
         break;
@@ -571,9 +576,10 @@ __device__ __forceinline__ void i8_body(const LaunchMaps *pm,
     int qslot = 0;
     uint32_t qph = 0;
     for (int it = 0;; ++it) {
-      const int tile = tq_get(tq, qslot, qph, err, true);
+      int ji;
+      const int tile = tq_get(tq, qslot, qph, ji, err, true);
       if (tile < 0) break;
-      const GemmJob &job = jobs[find_entry(jobs, njobs, tile, &GemmJob::tile_begin)];
+      const GemmJob &job = jobs[ji];
       const int local = tile - job.tile_begin;
       if (!mbar_wait(accfull, (uint32_t)(it & 1), err)) break;
       tc_fence_after();
