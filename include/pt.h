@@ -299,7 +299,12 @@ int libpt_rpt_dev_static(size_t oa, size_t va, const double *d_ov,
  * triples i<j (alpha), k (beta), and those of the beta-beta-alpha case
  * (unrestricted only) -- the order of src/pt.c:514-529.  Running every queue
  * entry once and calling libpt_plan_energy gives the solver's result
- * (including the restricted factor 2, src/pt.c:478).
+ * (including the restricted factor 2, src/pt.c:478): the same bits, but for
+ * restricted FP64 solves of v >= 48 whose same-spin blocks are the
+ * antisymmetrised mixed-spin ones to rounding.  The one-call entry points
+ * form the products those inputs share between the triples of {i, j, k}
+ * once; a plan, whose entries may run in any pieces, does not, and the two
+ * agree to rounding.
  *
  * kind: 0 = (T) restricted, 1 = (T) unrestricted, 2 = (fT) restricted,
  *       3 = (fT) unrestricted.
@@ -342,8 +347,8 @@ int libpt_plan_destroy(libpt_plan *plan);
  * the device, zero where another rank owns the entry -- with one in-place
  * sum all-reduce (ncclAllReduce, or MPI_Allreduce on a host copy), the
  * counterpart of the reference's one-double MPI_Allreduce (src/pt.c:
- * 474-477).  libpt_plan_energy on any rank then returns the one-GPU energy
- * bitwise: each slot holds exactly its owner's value, and the sum runs in
+ * 474-477).  libpt_plan_energy on any rank then returns the one-GPU plan's
+ * energy bitwise: each slot holds exactly its owner's value, and the sum runs in
  * queue order as for an unsharded solve. */
 
 /* Writes to idx (when non-NULL) the queue entries rank `rank` of `size`

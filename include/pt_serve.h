@@ -19,9 +19,12 @@
  *    others run joins the next round.  Rounds replay CUDA graphs captured
  *    once per set of kernel variants (the first round of a set launches
  *    directly and captures).
- *  - Each solve's energy is the same as libpt_plan / libpt_{r,u}{pt,ft}
- *    compute for it alone (per-triple energies in fixed order, summed in
- *    queue order): bitwise, whatever else shares its rounds.
+ *  - Each solve's energy is the same as libpt_plan computes for it alone
+ *    (per-triple energies in fixed order, summed in queue order): bitwise,
+ *    whatever else shares its rounds.  libpt_{r,u}{pt,ft} return the same
+ *    bits except for restricted FP64 inputs of v >= 48 whose same-spin
+ *    blocks are the antisymmetrised mixed-spin ones: those solves add the
+ *    same products in another order and agree to rounding.
  */
 #ifndef LIBPT_PT_SERVE_H
 #define LIBPT_PT_SERVE_H

@@ -25,9 +25,10 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
          "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 HOST_CXX = "/usr/bin/g++"   # the image's $CXX wrapper lacks some runtime specs
 
-SOURCES = ["gemm_dmma.cu", "gemm_tc.cu", "gemm_i8.cu", "epilogue.cu", "prep.cu",
+SOURCES = ["gemm_dmma.cu", "gemm_tc.cu", "gemm_i8.cu", "epilogue.cu", "epi_closed.cu",
+           "prep.cu",
            "exec.cu", "plan.cu", "plan_views.cu", "plan_upload.cu",
-           "plan_cases.cu", "plan_emu.cu", "plan_tune.cu", "plan_run.cu",
+           "plan_cases.cu", "plan_closed.cu", "plan_emu.cu", "plan_tune.cu", "plan_run.cu",
            "tune.cpp", "api.cpp", "noalloc.cu", "selftest.cu", "server.cpp",
            "producer.cu"]
 HEADERS = ["common.cuh", "engine.h", "exec.h", "plan.h", "plan_impl.h",

@@ -60,7 +60,7 @@ double host_solve(const char *name, int kind, size_t oa, size_t va, size_t ob,
   // OVVV copies streamed by occupied index next to the triples that need them
   int r = ptb::plan_create(kind, oa, va, ob, vb, args, dtype,
                            dtype ? mp_precision() : fp64_precision(), true, st,
-                           &p, nullptr, 0, 0, true);
+                           &p, nullptr, 0, 0, true, true);
   const double t1 = ptb::wall_seconds();
   if (!r) r = ptb::plan_run_streamed(p);
   if (!r) r = ptb::plan_energy(p, nullptr, 0, &e);
@@ -88,8 +88,9 @@ int dev_solve(int kind, size_t oa, size_t va, size_t ob, size_t vb,
   libpt_plan *p = nullptr;
   int r = ptb::plan_create(kind, oa, va, ob, vb, args, dtype,
                            dtype ? mp_precision() : fp64_precision(), false,
-                           static_cast<cudaStream_t>(stream), &p);
-  if (!r) r = ptb::plan_run(p, nullptr, p->queue.size());
+                           static_cast<cudaStream_t>(stream), &p, nullptr, 0,
+                           0, false, true);
+  if (!r) r = ptb::plan_run_solve(p);
   if (!r) r = ptb::plan_energy(p, nullptr, 0, e_out);
   ptb::plan_destroy(p);
   return r;

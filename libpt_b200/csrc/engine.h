@@ -105,6 +105,19 @@ cudaError_t gemm_dmma_launch(const GemmJob *d_jobs, GemmList *d_list,
                              int bm, int grid, unsigned *d_err,
                              cudaStream_t st);
 
+// Group jobs (closed-shell triples, plan_closed.cu): C[x][y][z] over v x v x v
+// with rows of pad4(v), M = N = v, ldc = v pad4(v); tiles of bm rows x
+// GRP_BY x GRP_BZ columns, numbered rows fastest, then z, then y.  A segment's
+// B operand is [k][y][z], or [k][z][y] where GRP_TR is set in its `neg`
+// (bit 0: subtract); bmap then names the view with the transposed box.
+constexpr int GRP_BY = 8, GRP_BZ = 16;
+constexpr int GRP_TR = 2;
+static_assert(GRP_BY * GRP_BZ == GEMM_BN, "a tile's columns");
+cudaError_t gemm_dmma_grp_launch(const GemmJob *d_jobs, GemmList *d_list,
+                                 int njobs, int ntiles, const LaunchMaps *pm,
+                                 int bm, int grid, unsigned *d_err,
+                                 cudaStream_t st);
+
 // ---- tensor-core (tcgen05) GEMM --------------------------------------------
 //
 // Operands as "planes" (e.g. TF32 hi / lo parts).  A planes: [P][Q][R][Kp]
@@ -243,6 +256,28 @@ cudaError_t epi_aab_launch(const EpiList *d_list, const EpiItem *d_items,
 int epi_blocks_per_sm(bool aab, bool ft);
 cudaError_t reduce_partials_launch(const RedList *d_list, int grid,
                                    cudaStream_t st);
+
+// ---- closed-shell triples (epi_closed.cu, plan_closed.cu) --------------------
+
+constexpr int GEPI_T = 8;                  // index block of a group's tiles
+constexpr int GEPI_THREADS = 6 * GEPI_T * GEPI_T;
+// Energies of groups {i < j < k}: items as for the epilogues above, args with
+// the three contraction outputs in offL / offR, ld[0] = v pad4(v), rowU1 =
+// pad4(v), tiles = blocks (X >= Y >= Z); partials [4][nblk]: the same-spin
+// triple, then the mixed-spin (ij;k), (ik;j), (jk;i).  grid = most tiles.
+cudaError_t epi_closed_launch(const EpiItem *d_items, bool ft, bool hasf,
+                              int grid, int nitems, cudaStream_t st);
+// Largest deviation (dst[0]) and magnitude (dst[1]), as bit patterns, of
+// same-spin matrices from the antisymmetrised mixed-spin ones; see
+// epi_closed.cu.
+cudaError_t closed_check_launch(const double *same, const double *mixed,
+                                int64_t nmat, int v, int64_t lds, int64_t ldm,
+                                bool packed, int o, bool partner,
+                                int64_t per_dst, unsigned long long *dst,
+                                cudaStream_t st);
+cudaError_t closed_check_oovo_launch(const double *same, const double *mixed,
+                                     int o, int64_t len,
+                                     unsigned long long *dst, cudaStream_t st);
 
 // ---- operand preparation ---------------------------------------------------
 

@@ -43,6 +43,10 @@ void Round::clear() {
       epi_blocks[a][f].clear();
       epi_hasf[a][f] = false;
     }
+  for (int f = 0; f < 2; ++f) {
+    grp[f].clear();
+    grp_hasf[f] = false;
+  }
   red.clear();
   gemm_flops = 0.0;
   triples = 0;
@@ -119,7 +123,7 @@ void Executor::destroy() {
 size_t Executor::bytes_for(size_t triples, size_t jobs_per_triple,
                            bool graphs) {
   const size_t jobs = triples * jobs_per_triple * sizeof(GemmJob);
-  return HDR + 64 * (EXEC_MAX_GROUPS + 5) +
+  return HDR + 64 * (EXEC_MAX_GROUPS + 7) +
          (graphs ? EXEC_MAX_GROUPS : 1) * jobs +
          triples * (sizeof(EpiItem) + sizeof(RedItem));
 }
@@ -165,6 +169,9 @@ int Executor::launch_all(const std::vector<GemmGroup> &groups,
       if (grp.kind == 0) {
         CK(gemm_dmma_launch(jobs, lst, njobs, ntiles, pm, grp.bm, grid, d_err,
                             st_));
+      } else if (grp.kind == 3) {
+        CK(gemm_dmma_grp_launch(jobs, lst, njobs, ntiles, pm, grp.bm, grid,
+                                d_err, st_));
       } else if (grp.kind == 1) {
         TcProducts pr;
         memset(&pr, 0, sizeof(pr));
@@ -203,6 +210,15 @@ int Executor::launch_all(const std::vector<GemmGroup> &groups,
       const EpiItem *items = fixed ? nullptr : epi_items_[a][f];
       CK(a ? epi_aab_launch(lst, items, f, hasf, grid, nitems, fixed, st_)
            : epi_aaa_launch(lst, items, f, hasf, grid, nitems, fixed, st_));
+      if (launches) ++*launches;
+    }
+  if (!fixed)
+    for (int f = 0; f < 2; ++f) {
+      if (r->grp[f].empty()) continue;
+      int grid = 0;
+      for (const EpiItem &it : r->grp[f]) grid = std::max(grid, it.nblk);
+      CK(epi_closed_launch(grp_items_[f], f, r->grp_hasf[f], grid,
+                           (int)r->grp[f].size(), st_));
       if (launches) ++*launches;
     }
   {
@@ -270,6 +286,15 @@ int Executor::run(Round &r, unsigned *d_err, ExecTiming *timing,
       eoff[a][f] = off;
       off = align64(off + r.epi[a][f].size() * sizeof(EpiItem));
     }
+  size_t grp_off[2];
+  for (int f = 0; f < 2; ++f) {
+    grp_off[f] = off;
+    off = align64(off + r.grp[f].size() * sizeof(EpiItem));
+  }
+  if (graphs_ && (!r.grp[0].empty() || !r.grp[1].empty())) {
+    set_error("executor: closed-shell groups need direct launches");
+    return LIBPT_ERR_ARG;
+  }
   const size_t roff = off;
   off = align64(off + r.red.size() * sizeof(RedItem));
   if (off > cap_) {
@@ -310,6 +335,11 @@ int Executor::run(Round &r, unsigned *d_err, ExecTiming *timing,
                              : it.back().block_begin + r.epi_blocks[a][f].back();
       std::memcpy(h + epi_slot(a, f), &l, sizeof(l));
     }
+  for (int f = 0; f < 2; ++f) {
+    std::memcpy(h + grp_off[f], r.grp[f].data(),
+                r.grp[f].size() * sizeof(EpiItem));
+    grp_items_[f] = reinterpret_cast<const EpiItem *>(d_buf_ + grp_off[f]);
+  }
   {
     std::memcpy(h + roff, r.red.data(), r.red.size() * sizeof(RedItem));
     RedList l;

@@ -19,7 +19,8 @@ namespace ptb {
 
 // One GEMM launch variant.
 struct GemmGroup {
-  int kind = 0;        // 0: FP64 DMMA, 1: 3xTF32, 2: emulated FP64 (INT8)
+  int kind = 0;        // 0: FP64 DMMA, 1: 3xTF32, 2: emulated FP64 (INT8),
+                       // 3: FP64 DMMA closed-shell groups
   int bm = 128;        // DMMA tile rows
   int slices = 0;      // INT8 digit planes
   I8Tile tile{0, 0};   // INT8 tile shape
@@ -46,6 +47,8 @@ struct Round {
   std::vector<EpiItem> epi[2][2];                   // [aab][ft], block_begin unset
   std::vector<int> epi_blocks[2][2];                // blocks of each item
   bool epi_hasf[2][2] = {};                         // some item's f_ov != 0
+  std::vector<EpiItem> grp[2];                      // closed-shell groups [ft]
+  bool grp_hasf[2] = {};                            // (direct launches only)
   std::vector<RedItem> red;
   double gemm_flops = 0.0;                          // reference flops
   size_t triples = 0;
@@ -103,6 +106,7 @@ class Executor {
   std::vector<const GemmJob *> gjobs_;   // device job arrays of the groups
   int epi_grid_[2][2] = {{0, 0}, {0, 0}};
   const EpiItem *epi_items_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+  const EpiItem *grp_items_[2] = {nullptr, nullptr};
 };
 
 }  // namespace ptb

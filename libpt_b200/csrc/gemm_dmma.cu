@@ -36,6 +36,17 @@
 // Tiles are numbered M-tile fastest inside a job and taken in order, so the
 // CTAs that share one B (OVVV) tile run at the same time and the tile is
 // fetched from DRAM once.
+// Group jobs (GRP; closed-shell triples, see plan_closed.cu) have columns
+// (y, z) over two virtual indices, and their B operands come in both orders:
+// [k][y][z], or [k][z][y] for a transposed segment.  A tile covers 8 y x 16 z
+// columns and its fragments run along the diagonals of 4 x 4 blocks of
+// (y, z): lane g of a fragment reads (y, z) = (g % 4, (g % 4 + s) % 4), s the
+// diagonal, so that of either layout
+//   [z/4][y][k][z%4]  (natural: one box of (4 z) x 16 k x 8 y x 4)
+//   [y/4][z][k][y%4]  (transposed: one box of (4 y) x 16 k x 16 z x 2)
+// a half-warp reads 16 different banks.  The sum of both orders therefore
+// needs no transposed copy of the integrals.  At the store two lanes exchange
+// half of their values so that each holds the four z of one y (32 bytes).
 #include "common.cuh"
 #include "engine.h"
 
@@ -94,7 +105,7 @@ __device__ __forceinline__ void mma_stage(double (&acc)[MF][4][4],
 // sub-partition hosts 3 of them, which bounds the kernel at 168 registers per
 // thread (16K registers per sub-partition); the 128-row tile's 64 FP64
 // accumulators per thread fit that without spilling.
-template <int BM, bool PM>
+template <int BM, bool PM, bool GRP>
 __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
                                           const GemmJob *__restrict__ jobs,
                                           const int njobs, const int ntiles,
@@ -141,7 +152,10 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
         const GemmJob &job = jobs[ji];
         const int local = tile - job.tile_begin;
         const int m0 = (local % job.mtiles) * BM;
-        const int n0 = (local / job.mtiles) * BN;
+        const int nb = local / job.mtiles;
+        const int n0 = nb * BN;
+        const int ntz = (job.N + GRP_BZ - 1) / GRP_BZ;   // GRP: N = v
+        const int y0 = (nb / ntz) * GRP_BY, z0 = (nb % ntz) * GRP_BZ;
         const int nseg = job.nseg;
         for (int s = 0; s < nseg && ok; ++s) {
           const GemmSeg sg = job.seg[s];
@@ -157,7 +171,12 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
             double *dB = sB + stage * BK * BN;
             const int k0 = ks * BK;
             tma_load_5d(dA, am, &full[stage], 0, m0, k0 / 4, sg.a_q, sg.a_p);
-            tma_load_4d(dB, bm, &full[stage], 0, k0, n0 / 4, sg.b_p);
+            if (!GRP)
+              tma_load_4d(dB, bm, &full[stage], 0, k0, n0 / 4, sg.b_p);
+            else if (sg.neg & GRP_TR)
+              tma_load_5d(dB, bm, &full[stage], 0, k0, z0, y0 / 4, sg.b_p);
+            else
+              tma_load_5d(dB, bm, &full[stage], 0, k0, y0, z0 / 4, sg.b_p);
             ++issued;
             if (++stage == ST) {
               stage = 0;
@@ -184,11 +203,19 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
   const int g = lane >> 2, t = lane & 3;
 
   // Per-lane fragment offsets inside one stage.
-  int boff[4];
+  int boff[4], bofft[4];   // bofft: transposed segments of group jobs
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
-    const int n = wn + 8 * h + g;
-    boff[h] = ((n >> 2) * BK + t) * 4 + (n & 3);
+    if (GRP) {
+      const int y = 4 * (h >> 1) + (g & 3);
+      const int z = 4 * (warp & 3) + ((g + 2 * (h & 1) + (g >> 2)) & 3);
+      boff[h] = (((z >> 2) * GRP_BY + y) * BK + t) * 4 + (z & 3);
+      bofft[h] = (((y >> 2) * GRP_BZ + z) * BK + t) * 4 + (y & 3);
+    } else {
+      const int n = wn + 8 * h + g;
+      boff[h] = ((n >> 2) * BK + t) * 4 + (n & 3);
+      bofft[h] = 0;
+    }
   }
 
   int stage = 0;
@@ -203,7 +230,7 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
     const GemmJob &job = jobs[ji];
     const int local = tile - job.tile_begin;
     const int m0 = (local % job.mtiles) * BM;
-    const int n0 = (local / job.mtiles) * BN;
+    const int nb = local / job.mtiles;
     const int nseg = job.nseg;
 
     double acc[MF][4][4];
@@ -222,8 +249,13 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
     const int aoff = (wm + g) * 4 + t;
 
     for (int s = 0; s < nseg && ok; ++s) {
+      const int neg = job.seg[s].neg;
       const unsigned long long mask =
-          job.seg[s].neg ? 0x8000000000000000ull : 0ull;
+          (GRP ? neg & 1 : neg) ? 0x8000000000000000ull : 0ull;
+      int bo[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        bo[h] = GRP && (neg & GRP_TR) ? bofft[h] : boff[h];
       const int nk = job.seg[s].ksteps, klast = job.seg[s].klast;
       for (int ks = 0; ks < nk; ++ks) {
         const int nkq = ks + 1 < nk ? BK / 4 : klast;
@@ -234,13 +266,13 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
         const double *A = sA + stage * BM * BK + aoff;
         const double *B = sB + stage * BK * BN;
         if (nf == MF)
-          mma_stage<MF, MF, BM>(acc, A, B, boff, mask, nkq);
+          mma_stage<MF, MF, BM>(acc, A, B, bo, mask, nkq);
         else if (nf == 1)
-          mma_stage<1, MF, BM>(acc, A, B, boff, mask, nkq);
+          mma_stage<1, MF, BM>(acc, A, B, bo, mask, nkq);
         else if (nf == 2)
-          mma_stage<2, MF, BM>(acc, A, B, boff, mask, nkq);
+          mma_stage<2, MF, BM>(acc, A, B, bo, mask, nkq);
         else if (MF == 4 && nf == 3)
-          mma_stage<3, MF, BM>(acc, A, B, boff, mask, nkq);
+          mma_stage<3, MF, BM>(acc, A, B, bo, mask, nkq);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == ST) {
@@ -255,6 +287,53 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
     double *const out = job.out;
     const int64_t ldc = job.ldc;
     const int M = job.M, N = job.N;
+    if (GRP) {
+      // lanes t and t ^ 2 hold diagonals 0, 2 and 1, 3 of the same two y:
+      // each keeps one y and takes its other two values from the partner
+      const int v4 = (N + 3) & ~3;
+      const int ntz = (N + GRP_BZ - 1) / GRP_BZ;
+      const int u = t >> 1, yy = 2 * (t & 1) + u;
+      const int z = (nb % ntz) * GRP_BZ + 4 * (warp & 3);
+      const bool odd = yy & 1, two = yy & 2;
+#pragma unroll
+      for (int f = 0; f < MF; ++f) {
+        if (f >= nf) break;   // uniform over the warp
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int r = m0 + wm + 16 * f + g + 8 * x;
+#pragma unroll
+          for (int yq = 0; yq < 2; ++yq) {
+            const double e0 = acc[f][2 * yq][2 * x],
+                         e1 = acc[f][2 * yq][2 * x + 1],
+                         o0 = acc[f][2 * yq + 1][2 * x],
+                         o1 = acc[f][2 * yq + 1][2 * x + 1];
+            const double re = __shfl_xor_sync(~0u, u ? e0 : e1, 2);
+            const double ro = __shfl_xor_sync(~0u, u ? o0 : o1, 2);
+            // diagonals 0..3 of this lane's y, then rotated to z order:
+            // diagonal s holds z % 4 = (yy + s) % 4
+            double d0 = u ? re : e0, d1 = u ? e1 : re, d2 = u ? ro : o0,
+                   d3 = u ? o1 : ro;
+            if (odd) {
+              const double w = d3;
+              d3 = d2;
+              d2 = d1;
+              d1 = d0;
+              d0 = w;
+            }
+            const double s0 = two ? d2 : d0, s1 = two ? d3 : d1,
+                         s2 = two ? d0 : d2, s3 = two ? d1 : d3;
+            const int y = (nb / ntz) * GRP_BY + 4 * yq + yy;
+            if (r < M && y < N && z < v4)
+              asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(
+                               out + (int64_t)r * ldc + y * v4 + z),
+                           "d"(s0), "d"(s1), "d"(s2), "d"(s3)
+                           : "memory");
+          }
+        }
+      }
+      continue;
+    }
+    const int n0 = nb * BN;
 #pragma unroll
     for (int f = 0; f < MF; ++f) {
       if (f >= nf) break;
@@ -280,14 +359,37 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_dmma_kernel(const __grid_constant__ LaunchMaps pm,
                      const GemmJob *__restrict__ jobs, int njobs, int ntiles,
                      GemmList *list, unsigned *err) {
-  dmma_body<BM, true>(&pm, jobs, njobs, ntiles, list, err);
+  dmma_body<BM, true, false>(&pm, jobs, njobs, ntiles, list, err);
 }
 
 template <int BM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_dmma_kernel_dm(const GemmJob *__restrict__ jobs, GemmList *list,
                         unsigned *err) {
-  dmma_body<BM, false>(nullptr, jobs, list->njobs, list->ntiles, list, err);
+  dmma_body<BM, false, false>(nullptr, jobs, list->njobs, list->ntiles, list, err);
+}
+
+// Group jobs (direct launches only).
+template <int BM>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+    gemm_dmma_grp_kernel(const __grid_constant__ LaunchMaps pm,
+                         const GemmJob *__restrict__ jobs, int njobs,
+                         int ntiles, GemmList *list, unsigned *err) {
+  dmma_body<BM, true, true>(&pm, jobs, njobs, ntiles, list, err);
+}
+
+template <int BM>
+cudaError_t launch_grp(const GemmJob *d_jobs, GemmList *d_list, int njobs,
+                       int ntiles, const LaunchMaps *pm, int grid,
+                       unsigned *d_err, cudaStream_t st) {
+  const size_t smem = gemm_smem_bytes(BM);
+  const cudaError_t e = cudaFuncSetAttribute(
+      gemm_dmma_grp_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (int)smem);
+  if (e != cudaSuccess) return e;
+  gemm_dmma_grp_kernel<BM><<<grid, GEMM_THREADS, smem, st>>>(
+      *pm, d_jobs, njobs, ntiles, d_list, d_err);
+  return cudaGetLastError();
 }
 
 template <int BM>
@@ -332,6 +434,17 @@ cudaError_t gemm_dmma_launch(const GemmJob *d_jobs, GemmList *d_list,
   if (bm == 96)
     return launch<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
   return launch<128>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+}
+
+cudaError_t gemm_dmma_grp_launch(const GemmJob *d_jobs, GemmList *d_list,
+                                 int njobs, int ntiles, const LaunchMaps *pm,
+                                 int bm, int grid, unsigned *d_err,
+                                 cudaStream_t st) {
+  if (grid <= 0) return cudaSuccess;
+  if (!pm) return cudaErrorInvalidValue;
+  if (bm == 96)
+    return launch_grp<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+  return launch_grp<128>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
 }
 
 }  // namespace ptb

@@ -90,10 +90,14 @@ LIBPT_API int libpt_rpt_dev_static(size_t oa, size_t va, const double *d_ov,
   if (int r = scratch_address(&base)) return r;
   const void *a[] = {d_ov, f_ov, t1, t2, i_oovo, i_oovv, i_ovvv};
   libpt_plan *p = nullptr;
+  // closed-shell groups take a little scratch of their own (views, tiles):
+  // only where the general plan leaves it
+  const bool solve = need + ((size_t)256 << 10) <=
+                     (size_t)LIBPT_STATIC_SCRATCH_BYTES;
   int r = ptb::plan_create(0, oa, va, oa, va, a, 0, LIBPT_PREC_FP64, false,
                            static_cast<cudaStream_t>(stream), &p, base,
-                           (size_t)LIBPT_STATIC_SCRATCH_BYTES);
-  if (!r) r = ptb::plan_run(p, nullptr, p->queue.size());
+                           (size_t)LIBPT_STATIC_SCRATCH_BYTES, 0, false, solve);
+  if (!r) r = ptb::plan_run_solve(p);
   if (!r) r = ptb::plan_energy(p, nullptr, 0, e_out);
   ptb::plan_destroy(p);
   return r;

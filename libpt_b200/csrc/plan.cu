@@ -47,7 +47,8 @@ const char *last_error() { return g_last_error.c_str(); }
 int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
                 const void *const *args, int dtype, int precision, bool host,
                 cudaStream_t st, libpt_plan **out, void *arena,
-                size_t arena_size, size_t arena_nb, bool stream_ovvv) {
+                size_t arena_size, size_t arena_nb, bool stream_ovvv,
+                bool solve) {
   *out = nullptr;
   if (kind < 0 || kind > 3 || dtype < 0 || dtype > 1 || !args) {
     set_error("libpt_plan_create: bad kind/dtype/args");
@@ -107,8 +108,14 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
   p->slices = slices;
   p->slices_store = slices;
   p->slices_auto = auto_slices && precision == LIBPT_PREC_EMU64;
+  // streamed when the blocks outgrow the staging buffers; smaller ones are
+  // copied first and run in full rounds (o = 8, v = 64: 25 MB take 0.6 ms to
+  // copy, and a round per index seven times the launches and partial waves)
   p->defer_ovvv = stream_ovvv && host && !unr && oa > 0 && va > 0 &&
-                  precision == LIBPT_PREC_FP64;
+                  precision == LIBPT_PREC_FP64 &&
+                  1.5 * (double)oa * (double)va * (double)va * (double)va *
+                          (dtype ? 4.0 : 8.0) >=
+                      2.0 * (double)PinnedRing::BYTES;
   if (const char *t = std::getenv("LIBPT_EMU_TOL")) {
     const double v = std::atof(t);
     if (v > 0) p->emu_tol = v;
@@ -171,6 +178,8 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
     p->up_stage[0] = up.stage[0];   // for the deferred OVVV copies
     p->up_stage[1] = up.stage[1];
     p->up_stage_bytes = up.stage_bytes;
+    p->closed_want = solve && closed_possible(p);
+    if (p->closed_want && (r = closed_check(p))) break;
     if (!g_dry && cudaStreamSynchronize(st) != cudaSuccess) {
       set_error(std::string("preparing operands: ") +
                 cudaGetErrorString(cudaGetLastError()));
@@ -192,8 +201,11 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
       }
       p->has_f = std::any_of(f.begin(), f.end(),
                              [](double x) { return x != 0.0; });
+      if (p->closed_want && (r = closed_read(p, st, p->deferred.empty() ? p->oa : 0)))
+        break;
     }
     if ((r = add_cases(p))) break;
+    if (p->closed_want && p->closed_on && (r = closed_build(p))) break;
     if (p->precision != LIBPT_PREC_FP64) {
       // the tensor-core paths read planes; of the padded FP64 blocks only the
       // amplitudes stay (the energy epilogue's disconnected term reads them)
@@ -290,10 +302,14 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
   }
   // deferred OVVV copies stay deferred only when nothing else in creation
   // reads them (the autotuner's probes would)
-  if (!r && !p->deferred.empty() && tune_would_probe(p)) r = flush_deferred(p);
+  // (a solve that runs closed-shell groups is not probed: few of its triples
+  // run the general jobs the probes would time)
+  const bool tune = !p->closed_on;
+  if (!r && tune && !p->deferred.empty() && tune_would_probe(p))
+    r = flush_deferred(p);
   const double t_tune = wall_seconds();
   if (!r && !g_dry && p->slices_auto) r = choose_slices(p);
-  if (!r && !g_dry) r = autotune(p);
+  if (!r && !g_dry && tune) r = autotune(p);
   p->prof_tune = wall_seconds() - t_tune;
   if (r) {
     plan_destroy(p);
@@ -351,7 +367,9 @@ void plan_destroy(libpt_plan *p) {
     cudaStreamSynchronize(p->st_up);
     cudaStreamDestroy(p->st_up);
   }
-  if (p->ev_up) cudaEventDestroy(p->ev_up);
+  for (cudaEvent_t e : p->ev_up)
+    if (e) cudaEventDestroy(e);
+  if (p->st_rd) cudaStreamDestroy(p->st_rd);
   p->tm.clear();
   if (p->exec_ready) p->exec.destroy();
   for (void *a : p->allocs) cudaFree(a);

@@ -130,7 +130,8 @@ struct libpt_plan {
   bool defer_ovvv = false;   // record host OVVV copies instead of making them
   std::vector<DeferredBlock> deferred;
   cudaStream_t st_up = nullptr;
-  cudaEvent_t ev_up = nullptr;
+  cudaEvent_t ev_up[2] = {nullptr, nullptr};
+  cudaStream_t st_rd = nullptr;   // reads the rows' closed-shell checks
   void *up_stage[2] = {nullptr, nullptr};
   size_t up_stage_bytes = 0;
   std::vector<void *> allocs;
@@ -179,19 +180,27 @@ struct libpt_plan {
   bool timing = false;
   ptb::ExecTiming tm;
   int64_t launches = 0;                      // kernels launched by runs
+  // closed-shell groups of a restricted one-call solve (plan_closed.cu)
+  bool closed_want = false;                  // created for plan_run_solve
+  bool closed_on = false;                    // the relations hold
+  std::vector<char> closed_ok;               // ... of each occupied index
+  unsigned long long *closed_words = nullptr;   // measured, device
+  ptb::SpinCase closed;
 };
 
 namespace ptb {
 
 // args: pt.h tensors of `kind` in the reference's order; `host` selects host
 // (true) or device (false) pointers; dtype 0 = FP64, 1 = FP32.
+// solve: the plan is for one plan_run_solve / plan_run_streamed of its whole
+// queue, which may run closed-shell groups.
 // arena: carve every device buffer from [arena, arena + arena_size) (no
 // allocation); arena_nb caps the triples of one round (0: what fits).
 int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
                 const void *const *args, int dtype, int precision, bool host,
                 cudaStream_t st, libpt_plan **out, void *arena = nullptr,
                 size_t arena_size = 0, size_t arena_nb = 0,
-                bool stream_ovvv = false);
+                bool stream_ovvv = false, bool solve = false);
 // Exact device bytes plan_create takes from an arena for these arguments
 // with rounds of up to nb triples (a sizing pass: host logic only, no
 // device work); 0 if the arguments are invalid.
@@ -216,6 +225,9 @@ int dmma_map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R,
 int dmma_map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld,
                int64_t K, int64_t P);
 int plan_run(libpt_plan *p, const int64_t *idx, size_t n);
+// The whole queue of a plan created for it (`solve`): closed-shell groups
+// where the inputs allow, else as plan_run.
+int plan_run_solve(libpt_plan *p);
 // The whole queue; with deferred OVVV copies, each occupied index's rows are
 // copied on a second stream while the triples whose indices are all below it
 // run (same energies: each triple writes its own slot).

@@ -334,7 +334,7 @@ int build_aab(libpt_plan *p, SpinCase &c) {
 // and a tile cannot run faster than its operands arrive (26 bytes per cycle
 // with 32-byte TMA box rows).  Only a last tile of 16 rows is bound by its
 // operands, so 97..112 rows go to one 128-row tile, not to 96 + 16.
-static int64_t dmma_row_cost(int64_t m, int64_t bm) {
+int64_t dmma_row_cost(int64_t m, int64_t bm) {
   int64_t cost = 0;
   for (int64_t r = 0; r < m; r += bm) {
     const int64_t rows = (std::min(bm, m - r) + 15) / 16 * 16;

@@ -37,6 +37,9 @@ int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
           int64_t P, int bm);
 int map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld, int64_t K,
           int64_t P);
+// Any FP64 view (rank <= 5, strides in bytes from dimension 1 on).
+int map_f64(CUtensorMap *m, const double *p, int rank, const int64_t *dims,
+            const int64_t *strides, const int *box);
 // Tensor-core views of a case: TF32 plane pairs at map indices 2i, 2i+1.
 int build_tc(libpt_plan *p, SpinCase &c);
 
@@ -181,6 +184,9 @@ int flush_deferred(libpt_plan *p);
 
 // ---- spin cases, job templates, queue (plan_cases.cu) -----------------------
 int add_cases(libpt_plan *p);
+SegT seg(int amap, int bmap, bool neg, int aq, int ap, int bp, int64_t k);
+// Modelled cost of m rows in DMMA tiles of bm rows.
+int64_t dmma_row_cost(int64_t m, int64_t bm);
 // Copies each case's kernel views (tensor maps) and epilogue arguments to
 // device memory, where the kernels read them.  Re-run after any map change.
 int upload_views(libpt_plan *p);
@@ -198,9 +204,27 @@ bool tune_would_probe(libpt_plan *p);
 int autotune(libpt_plan *p);
 
 // ---- rounds (plan_run.cu) ---------------------------------------------------
-// Sizes the round resources for `ents` (up to the workspace budget).
-int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents);
+// Sizes the round resources for `ents` and `groups` closed-shell groups (up
+// to the workspace budget).
+int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
+                    size_t groups = 0);
 // Runs queue entries in rounds, each filling the plan's round resources.
 int run_entries(libpt_plan *p, const std::vector<int64_t> &ents);
+
+// ---- closed-shell triples (plan_closed.cu) ----------------------------------
+// Smallest v whose restricted solves run groups.
+constexpr int CLOSED_MIN_V = 48;
+bool closed_possible(const libpt_plan *p);
+int closed_build(libpt_plan *p);
+int closed_check(libpt_plan *p);
+int closed_check_ovvv(libpt_plan *p, int i0, int i1, cudaStream_t s);
+// Reads the measured relations on stream s and decides closed_on, and
+// closed_ok of the occupied indices below `upto`.
+int closed_read(libpt_plan *p, cudaStream_t s, int upto);
+void closed_split(const libpt_plan *p, int lo, int hi,
+                  std::vector<int4> &groups, std::vector<int64_t> &rest);
+int closed_run(libpt_plan *p, const std::vector<int4> &groups,
+               const std::vector<int64_t> &rest);
+bool closed_fits(const libpt_plan *p);
 
 }  // namespace ptb

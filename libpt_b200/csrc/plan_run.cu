@@ -20,8 +20,18 @@ namespace ptb {
 // Sizes the round resources for `ents` (up to the workspace budget): the
 // contraction outputs of every triple, their partial energies and the
 // round descriptors.
-int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents) {
+int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
+                    size_t groups) {
   int64_t want = 0, biggest = 0;
+  int64_t small = p->ws_stride_min;   // least workspace of a triple
+  int ntiles = p->ntiles_max;
+  if (groups) {
+    const int64_t st = p->closed.ws_stride;
+    biggest = st;
+    want = (int64_t)std::min<size_t>(groups, p->ws_budget / 8 / st + 1) * st;
+    small = std::min(small, st / 4);
+    ntiles = std::max(ntiles, p->closed.ntiles);
+  }
   for (int64_t q : ents) {
     const int64_t st = p->cases[p->queue[q].x].ws_stride;
     want += st;
@@ -35,9 +45,12 @@ int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents) {
   }
   want = std::max(std::min<int64_t>(want, (int64_t)(p->ws_budget / 8)), biggest);
   const size_t tri = std::max<size_t>(
-      1, std::min<size_t>({(size_t)4096, ents.size(),
-                           (size_t)(want / std::max<int64_t>(p->ws_stride_min, 1))}));
-  if (want <= p->ws_cap && tri <= p->tri_cap) return LIBPT_OK;
+      groups ? 4 : 1,
+      std::min<size_t>({(size_t)4096, ents.size() + 4 * groups,
+                        (size_t)(want / std::max<int64_t>(small, 1))}));
+  if (want <= p->ws_cap && tri <= p->tri_cap &&
+      (int64_t)tri * ntiles <= p->part_cap)
+    return LIBPT_OK;
   CK(cudaStreamSynchronize(p->st));
   for (void **q : {(void **)&p->ws, (void **)&p->partials, (void **)&p->d_desc}) {
     if (!*q) continue;
@@ -52,7 +65,7 @@ int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents) {
   }
   p->ws_cap = p->part_cap = 0;
   p->tri_cap = 0;
-  const int64_t part = (int64_t)tri * std::max(p->ntiles_max, 1);
+  const int64_t part = (int64_t)tri * std::max(ntiles, 1);
   const size_t desc = Executor::bytes_for(tri, p->jobs_max);
   if (dalloc(p, (void **)&p->ws, want * 8) ||
       dalloc(p, (void **)&p->partials, part * 8) ||

@@ -192,7 +192,7 @@ int flush_deferred(libpt_plan *p) {
 
 int plan_run_streamed(libpt_plan *p) {
   const size_t total = p->queue.size();
-  if (p->deferred.empty()) return plan_run(p, nullptr, total);
+  if (p->deferred.empty()) return plan_run_solve(p);
   if (g_dry) return LIBPT_OK;
   // triples by the largest occupied index they read (every OVVV row a
   // triple (i, j, k) reads belongs to i, j or k)
@@ -206,10 +206,18 @@ int plan_run_streamed(libpt_plan *p) {
   }
   // round resources for the whole queue first: growing them later would
   // wait for the triples already running
-  if (int r = ensure_capacity(p, all)) return r;
+  if (p->closed_on && ensure_capacity(p, all, total / 4 + 1) != LIBPT_OK) {
+    cudaGetLastError();   // a group's outputs do not fit: general jobs
+    p->closed_on = false;
+  }
+  if (!p->closed_on)
+    if (int r = ensure_capacity(p, all)) return r;
   if (!p->st_up) {
     CK(cudaStreamCreateWithFlags(&p->st_up, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&p->ev_up, cudaEventDisableTiming));
+    for (cudaEvent_t &e : p->ev_up)
+      CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (p->closed_on)
+      CK(cudaStreamCreateWithFlags(&p->st_rd, cudaStreamNonBlocking));
   }
   Uploader up{p, true, p->dtype == 1};
   up.stage[0] = p->up_stage[0];
@@ -217,8 +225,23 @@ int plan_run_streamed(libpt_plan *p) {
   up.stage_bytes = p->up_stage_bytes;
   up.s = p->st_up;
   // the copies start after everything plan creation queued on its stream
-  CK(cudaEventRecord(p->ev_up, p->st));
-  CK(cudaStreamWaitEvent(p->st_up, p->ev_up, 0));
+  CK(cudaEventRecord(p->ev_up[0], p->st));
+  CK(cudaStreamWaitEvent(p->st_up, p->ev_up[0], 0));
+  // the triples of index m, once its rows (event m % 2) are on the device;
+  // closed-shell solves first read whether the rows satisfy the relation
+  std::vector<int4> groups;
+  std::vector<int64_t> rest;
+  auto launch = [&](int m) -> int {
+    CK(cudaStreamWaitEvent(p->st, p->ev_up[m & 1], 0));
+    if (by_index[(size_t)m].empty()) return LIBPT_OK;
+    if (!p->closed_on) return run_entries(p, by_index[(size_t)m]);
+    CK(cudaEventSynchronize(p->ev_up[m & 1]));
+    if (int r = closed_read(p, p->st_rd, m + 1)) return r;
+    groups.clear();
+    rest.clear();
+    closed_split(p, m, m + 1, groups, rest);
+    return closed_run(p, groups, rest);
+  };
   const size_t es = p->dtype ? 4 : 8;
   for (int m = 0; m < o; ++m) {
     for (const DeferredBlock &d : p->deferred) {
@@ -227,11 +250,19 @@ int plan_run_streamed(libpt_plan *p) {
                          d.rows_per_index, d.w, d.dpitch))
         return r;
     }
-    CK(cudaEventRecord(p->ev_up, p->st_up));
-    CK(cudaStreamWaitEvent(p->st, p->ev_up, 0));
-    if (!by_index[(size_t)m].empty())
-      if (int r = run_entries(p, by_index[(size_t)m])) return r;
+    if (p->closed_on)
+      if (int r = closed_check_ovvv(p, m, m + 1, p->st_up)) return r;
+    CK(cudaEventRecord(p->ev_up[m & 1], p->st_up));
+    // closed-shell solves wait on the host for a row's check: they launch an
+    // index after the next one's rows are queued, so the copies stay busy
+    if (!p->closed_on) {
+      if (int r = launch(m)) return r;
+    } else if (m > 0) {
+      if (int r = launch(m - 1)) return r;
+    }
   }
+  if (p->closed_on)
+    if (int r = launch(o - 1)) return r;
   p->deferred.clear();
   return LIBPT_OK;
 }

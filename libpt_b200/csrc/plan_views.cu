@@ -34,6 +34,33 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// FP64 view of any rank without swizzle; out-of-range elements read zero.
+int map_f64(CUtensorMap *m, const double *p, int rank, const int64_t *dims,
+            const int64_t *strides, const int *box) {
+  if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled unavailable");
+    return LIBPT_ERR_CUDA;
+  }
+  cuuint64_t d[5], s[4];
+  cuuint32_t b[5], es[5] = {1, 1, 1, 1, 1};
+  for (int x = 0; x < rank; ++x) {
+    d[x] = (cuuint64_t)std::max<int64_t>(dims[x], 1);
+    b[x] = (cuuint32_t)box[x];
+    if (x + 1 < rank) s[x] = (cuuint64_t)strides[x];
+  }
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rank, (void *)p, d, s, b,
+                   es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled (FP64 view) failed: " + std::to_string(r));
+    return LIBPT_ERR_CUDA;
+  }
+  return LIBPT_OK;
+}
+
 // A-view of a padded block [P][Q][R][Kpad] with logical K: dims
 // (4, R, Kpad/4, Q, P), box (4, bm, GEMM_BK/4, 1, 1), which lands in shared
 // memory as [k/4][m][k%4].  K is split in fours so that one TMA copy brings
@@ -41,30 +68,11 @@ EncodeTiledFn encode_fn() {
 // of copies, not by bytes (see gemm_dmma.cu).  The pad columns hold zeros.
 int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
           int64_t P, int bm) {
-  if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
-  EncodeTiledFn enc = encode_fn();
-  if (!enc) {
-    set_error("cuTensorMapEncodeTiled unavailable");
-    return LIBPT_ERR_CUDA;
-  }
   const int64_t kp = pad4(std::max<int64_t>(K, 1));
-  cuuint64_t dims[5] = {4, (cuuint64_t)std::max<int64_t>(R, 1),
-                        (cuuint64_t)(kp / 4),
-                        (cuuint64_t)std::max<int64_t>(Q, 1),
-                        (cuuint64_t)std::max<int64_t>(P, 1)};
-  cuuint64_t strides[4] = {(cuuint64_t)(kp * 8), 32, (cuuint64_t)(R * kp * 8),
-                           (cuuint64_t)(Q * R * kp * 8)};
-  cuuint32_t box[5] = {4, (cuuint32_t)bm, GEMM_BK / 4, 1, 1};
-  cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, (void *)p, dims,
-                   strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled (A view) failed: " + std::to_string(r));
-    return LIBPT_ERR_CUDA;
-  }
-  return LIBPT_OK;
+  const int64_t dims[5] = {4, R, kp / 4, Q, P};
+  const int64_t strides[4] = {kp * 8, 32, R * kp * 8, Q * R * kp * 8};
+  const int box[5] = {4, bm, GEMM_BK / 4, 1, 1};
+  return map_f64(m, p, 5, dims, strides, box);
 }
 
 // B-view of a padded block [P][K][Nld] with logical N (a multiple of 4):
@@ -72,28 +80,10 @@ int map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R, int64_t Q,
 // which lands in shared memory as [n/4][k][n%4].
 int map_b(CUtensorMap *m, const double *p, int64_t N, int64_t Nld, int64_t K,
           int64_t P) {
-  if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
-  EncodeTiledFn enc = encode_fn();
-  if (!enc) {
-    set_error("cuTensorMapEncodeTiled unavailable");
-    return LIBPT_ERR_CUDA;
-  }
-  cuuint64_t dims[4] = {4, (cuuint64_t)std::max<int64_t>(K, 1),
-                        (cuuint64_t)std::max<int64_t>(pad4(N) / 4, 1),
-                        (cuuint64_t)std::max<int64_t>(P, 1)};
-  cuuint64_t strides[3] = {(cuuint64_t)(Nld * 8), 32,
-                           (cuuint64_t)(K * Nld * 8)};
-  cuuint32_t box[4] = {4, (cuuint32_t)GEMM_BK, GEMM_BN / 4, 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void *)p, dims,
-                   strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled (B view) failed: " + std::to_string(r));
-    return LIBPT_ERR_CUDA;
-  }
-  return LIBPT_OK;
+  const int64_t dims[4] = {4, K, pad4(N) / 4, P};
+  const int64_t strides[3] = {Nld * 8, 32, K * Nld * 8};
+  const int box[4] = {4, GEMM_BK, GEMM_BN / 4, 1};
+  return map_f64(m, p, 4, dims, strides, box);
 }
 
 int tc_encode(CUtensorMap *m, const float *p, int rank, const cuuint64_t *dims,

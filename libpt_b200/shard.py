@@ -6,7 +6,7 @@ queue with q % size == rank, and the ranks exchange once.  The reference
 all-reduces one double; here the exchange is a sum all-reduce of the
 per-triple energy slots (queue_length doubles, zero where another rank owns
 the entry), after which every rank sums them in queue order and returns the
-one-GPU energy bitwise.  NCCL moves the slots GPU to GPU (NVLink); with
+one-GPU plan's energy bitwise.  NCCL moves the slots GPU to GPU (NVLink); with
 gloo the same function runs on host tensors.
 """
 import torch
