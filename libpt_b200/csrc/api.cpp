@@ -4,6 +4,8 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
+#include <vector>
 
 #include "plan.h"
 #include "pt.h"
@@ -44,13 +46,52 @@ int fp64_precision() {
   abort();
 }
 
+// Streams of the host-pointer solves, kept between calls (creating and
+// destroying one takes 0.15 to 0.8 ms): at most four idle ones a process,
+// each used by one call at a time.
+struct IdleStream {
+  int dev;
+  cudaStream_t st;
+};
+std::mutex g_stream_mu;
+std::vector<IdleStream> g_idle_streams;
+
+bool take_stream(cudaStream_t *st, int *dev) {
+  if (cudaGetDevice(dev) != cudaSuccess) return false;
+  {
+    std::lock_guard<std::mutex> g(g_stream_mu);
+    for (size_t x = 0; x < g_idle_streams.size(); ++x)
+      if (g_idle_streams[x].dev == *dev) {
+        *st = g_idle_streams[x].st;
+        g_idle_streams.erase(g_idle_streams.begin() + x);
+        // a device reset since then took the stream with it
+        if (cudaStreamQuery(*st) == cudaSuccess) return true;
+        cudaGetLastError();
+        break;
+      }
+  }
+  return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking) == cudaSuccess;
+}
+
+void give_stream(cudaStream_t st, int dev) {
+  {
+    std::lock_guard<std::mutex> g(g_stream_mu);
+    if (g_idle_streams.size() < 4) {
+      g_idle_streams.push_back({dev, st});
+      return;
+    }
+  }
+  cudaStreamDestroy(st);
+}
+
 // Host-pointer solve: stage the caller's arrays to the current device, run
 // every triple, return the energy.  Aborts on failure like the reference
 // (src/pt.c:208-209).
 double host_solve(const char *name, int kind, size_t oa, size_t va, size_t ob,
                   size_t vb, const void *const *args, int dtype) {
+  int dev = 0;
   cudaStream_t st = nullptr;
-  if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
+  if (!take_stream(&st, &dev)) {
     ptb::set_error(cudaGetErrorString(cudaGetLastError()));
     fatal(name);
   }
@@ -73,7 +114,7 @@ double host_solve(const char *name, int kind, size_t oa, size_t va, size_t ob,
             p->prof_tune, t1 - t0, ptb::wall_seconds() - t1, p->precision,
             p->precision == LIBPT_PREC_EMU64 ? p->slices : 0);
   ptb::plan_destroy(p);
-  cudaStreamDestroy(st);
+  give_stream(st, dev);
   if (r) fatal(name);
   return e;
 }
@@ -357,6 +398,7 @@ LIBPT_API int libpt_plan_energy_slots(libpt_plan *plan, double **slots) {
     ptb::set_error("libpt_plan_energy_slots: NULL argument");
     return LIBPT_ERR_ARG;
   }
+  plan->slots_shared = true;
   *slots = plan->e_slot;
   return LIBPT_OK;
 }

@@ -220,11 +220,7 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
                            &set->oovo[2], &set->oovo[3], &set->taup[0],
                            &set->taup[1]}) {
           if (!*q) continue;
-          auto it = std::find(p->allocs.begin(), p->allocs.end(), (void *)*q);
-          if (it != p->allocs.end()) {
-            cudaFree(*q);
-            p->allocs.erase(it);
-          }
+          dfree(p, *q);
         }
     }
     if ((r = dalloc(p, (void **)&p->e_slot, (p->queue.size() + 1) * 8))) break;
@@ -289,12 +285,7 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
       p->ws_budget = nb * p->ws_stride * 8;
       break;
     }
-    // workspace budget: half of what is free, between 64 MiB and 16 GiB;
-    // the buffers themselves are sized by the first run that needs them
-    size_t fr = 0, tot = 0;
-    cudaMemGetInfo(&fr, &tot);
-    p->ws_budget = std::min<size_t>(std::max<size_t>(fr / 2, (size_t)64 << 20),
-                                    (size_t)16 << 30);
+    // (the round buffers are sized by the first run that needs them)
   } while (0);
   if (!r && !g_dry && profile_enabled()) {
     cudaStreamSynchronize(st);
@@ -372,7 +363,9 @@ void plan_destroy(libpt_plan *p) {
   if (p->st_rd) cudaStreamDestroy(p->st_rd);
   p->tm.clear();
   if (p->exec_ready) p->exec.destroy();
-  for (void *a : p->allocs) cudaFree(a);
+  // the caller may read the energy slots on streams of its own
+  if (p->slots_shared) cudaDeviceSynchronize();
+  while (!p->allocs.empty()) dfree(p, p->allocs.back());
   delete p;
 }
 

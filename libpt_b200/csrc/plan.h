@@ -134,7 +134,8 @@ struct libpt_plan {
   cudaStream_t st_rd = nullptr;   // reads the rows' closed-shell checks
   void *up_stage[2] = {nullptr, nullptr};
   size_t up_stage_bytes = 0;
-  std::vector<void *> allocs;
+  std::vector<void *> allocs;           // device buffers (no arena)
+  std::vector<void *> pooled;           // ... those of the library's pool
   ptb::OperandSet L, R;
   double *d_ov = nullptr, *ov1 = nullptr, *ov2 = nullptr;
   bool has_f = true;                    // f_ov / f2_ov not all zero
@@ -151,7 +152,9 @@ struct libpt_plan {
   char *d_desc = nullptr;
   int64_t ws_cap = 0, part_cap = 0;     // doubles held
   size_t tri_cap = 0;                   // triples a round may hold
-  size_t ws_budget = 0;                 // workspace size limit (bytes)
+  size_t ws_budget = 0;                 // workspace size limit (bytes; 0:
+                                        // not measured yet)
+  bool slots_shared = false;            // libpt_plan_energy_slots was called
   int64_t ws_stride = 0;                // max over cases (doubles)
   int64_t ws_stride_min = 0;            // min over cases (doubles)
   int ntiles_max = 0;                   // max epilogue tiles of a triple

@@ -22,41 +22,60 @@ namespace ptb {
 // round descriptors.
 int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
                     size_t groups) {
-  int64_t want = 0, biggest = 0;
+  int64_t biggest = 0;
+  double total = 0.0;                 // outputs of everything to run (doubles)
   int64_t small = p->ws_stride_min;   // least workspace of a triple
   int ntiles = p->ntiles_max;
   if (groups) {
     const int64_t st = p->closed.ws_stride;
     biggest = st;
-    want = (int64_t)std::min<size_t>(groups, p->ws_budget / 8 / st + 1) * st;
+    total = (double)groups * (double)st;
     small = std::min(small, st / 4);
     ntiles = std::max(ntiles, p->closed.ntiles);
   }
   for (int64_t q : ents) {
     const int64_t st = p->cases[p->queue[q].x].ws_stride;
-    want += st;
+    total += (double)st;
     biggest = std::max(biggest, st);
-    if (want * 8 >= (int64_t)p->ws_budget) break;
+  }
+  // The workspace of a round: allocating and freeing it costs up to 1.4 ms
+  // per GB, each round some 50 us of launches and a partial last wave, so the
+  // sum is least near 0.19 sqrt(outputs in GB) GB; at least 1 GiB (a round of
+  // that size is long enough), at most the budget.  (o = 14, v = 143, 47 GB
+  // of outputs: 24 ms of the solve went to a 16 GiB workspace.)
+  double want_all = std::min(
+      total, std::max((double)((size_t)1 << 30), 0.19e9 * std::sqrt(total * 8e-9)) / 8);
+  // beyond 2 GiB: no more than half of what is free, nor than 16 GiB (the
+  // query itself can take milliseconds; smaller workspaces are halved below
+  // where they do not fit)
+  if (!p->arena && want_all * 8 > (double)((size_t)2 << 30)) {
+    if (!p->ws_budget) {
+      size_t fr = 0, tot = 0;
+      cudaMemGetInfo(&fr, &tot);
+      p->ws_budget = std::min<size_t>(std::max(fr / 2, (size_t)64 << 20),
+                                      (size_t)16 << 30);
+    }
+    want_all = std::min(want_all, (double)(p->ws_budget / 8));
   }
   if (p->arena) {   // fixed resources: rounds are cut to what they hold
     if (p->tri_cap >= 1 && biggest <= p->ws_cap) return LIBPT_OK;
     set_error("scratch arena workspace smaller than one triple");
     return LIBPT_ERR_NOMEM;
   }
-  want = std::max(std::min<int64_t>(want, (int64_t)(p->ws_budget / 8)), biggest);
-  const size_t tri = std::max<size_t>(
-      groups ? 4 : 1,
-      std::min<size_t>({(size_t)4096, ents.size() + 4 * groups,
-                        (size_t)(want / std::max<int64_t>(small, 1))}));
-  if (want <= p->ws_cap && tri <= p->tri_cap &&
-      (int64_t)tri * ntiles <= p->part_cap)
+  auto triples = [&](int64_t w) {
+    return std::max<size_t>(
+        groups ? 4 : 1,
+        std::min<size_t>({(size_t)4096, ents.size() + 4 * groups,
+                          (size_t)(w / std::max<int64_t>(small, 1))}));
+  };
+  int64_t want = std::max((int64_t)want_all, biggest);
+  if (want <= p->ws_cap && triples(want) <= p->tri_cap &&
+      (int64_t)triples(want) * ntiles <= p->part_cap)
     return LIBPT_OK;
   CK(cudaStreamSynchronize(p->st));
   for (void **q : {(void **)&p->ws, (void **)&p->partials, (void **)&p->d_desc}) {
     if (!*q) continue;
-    auto it = std::find(p->allocs.begin(), p->allocs.end(), *q);
-    if (it != p->allocs.end()) p->allocs.erase(it);
-    cudaFree(*q);
+    dfree(p, *q);
     *q = nullptr;
   }
   if (p->exec_ready) {
@@ -65,10 +84,14 @@ int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
   }
   p->ws_cap = p->part_cap = 0;
   p->tri_cap = 0;
+  while (dalloc(p, (void **)&p->ws, want * 8)) {
+    if (want == biggest) return LIBPT_ERR_NOMEM;
+    want = std::max(want / 2, biggest);
+  }
+  const size_t tri = triples(want);
   const int64_t part = (int64_t)tri * std::max(ntiles, 1);
   const size_t desc = Executor::bytes_for(tri, p->jobs_max);
-  if (dalloc(p, (void **)&p->ws, want * 8) ||
-      dalloc(p, (void **)&p->partials, part * 8) ||
+  if (dalloc(p, (void **)&p->partials, part * 8) ||
       dalloc(p, (void **)&p->d_desc, desc))
     return LIBPT_ERR_NOMEM;
   if (int r = p->exec.init(p->st, p->d_desc, desc, false)) return r;
