@@ -11,11 +11,23 @@
 // Energy per element: (W - X) * R / D with R = W for (T) and R = the right
 // amplitude for (fT); X is the disconnected term, D the denominator.
 //
-// A CTA handles an 8 (a) x 8 (b) x 32 (c) tile of one triple; lanes run over
-// c so the loads of U1/T rows are coalesced, and the operands that are
-// contiguous in a or b (T[c][ab], U2, P) are staged through shared memory
-// as [x][y][c] rows of EPI_CS = 34 doubles: the fill (8 consecutive y per
-// 8 lanes) and the reads (32 consecutive c) are both free of bank conflicts.
+// A CTA handles an 8 (a) x 8 (b) x 32 (c) tile of one triple; warp w takes
+// a = a0 + w, lane l takes c = c0 + l, and a thread the tile's 8 values of b.
+// U1 and T rows are read along c (coalesced).  The operands that are
+// contiguous in b or a (T[c][ab], U2, P) are needed as runs of 8 doubles per
+// (a, c) or (b, c):
+//   (T)   copied to shared memory with cp.async, which holds no registers, so
+//         all of a tile's loads are in flight together: mixed-spin runs by 8
+//         lanes each into [row][x][c] with rows of EPI_CS doubles (copies and
+//         reads free of bank conflicts), same-spin runs 16 bytes a copy, as
+//         the five aligned pairs that cover pair(a, b0) .. + 7;
+//   (fT)  twice the operands: that staging leaves one mixed-spin CTA an SM.
+//         Runs are read 32 bytes a load into the thread that needs them, and
+//         only U2[b][c][a], which belongs to the eight warps, is staged.
+// Measured (v = 180): mixed-spin (fT) 2.9 -> 2.0 ms with the direct loads;
+// (T) with them 1.04 ms against 0.95 ms staged (24 triples of v = 201), and
+// 16-byte copies of the mixed-spin runs 1.15 ms (they spread a copy over more
+// rows and double the bank cycles of the reads).
 // Each CTA tile writes one partial sum; reduce_partials adds them in a fixed
 // order.  Launches are persistent: a fixed grid strides over the flat tiles
 // of a device-memory item list (EpiList), whose items (triples) may belong
@@ -28,26 +40,28 @@ namespace ptb {
 
 namespace {
 
-// CTAs per SM the energy kernels are compiled for (80 registers each): the
-// kernels are latency-bound, and three CTAs of 256 threads keep more loads
-// in flight than two (31 -> 40 % of DRAM peak measured), four spill.
-constexpr int EPI_MINB = 3;
+// CTAs per SM the energy kernels are compiled for.  (T): three, of 80
+// registers; the kernels are latency-bound, and three CTAs of 256 threads keep
+// more loads in flight than two (31 -> 40 % of DRAM peak measured), four
+// spill.  (fT): two, of 128 registers, which hold a thread's operand runs
+// (v = 180: 2.02 ms with two, 2.20 ms with three and spills).
+constexpr int epi_minb(bool ft) { return ft ? 2 : 3; }
 
 // Shared-memory layout (doubles) of the mixed-spin epilogue's staged
-// disconnected-term slices, after its U2 / P staging: g1[j,k][b][c],
+// disconnected-term slices, after its U2 staging: g1[j,k][b][c],
 // g1[i,k][b][c] (EPI_B x EPI_C each), g1[j,i][b][a] (EPI_B x EPI_A), t1[i][b],
 // t1[j][b], d[j][b] (EPI_B each), then the same for the f_ov half.
 constexpr int EPI_SD_G1JK = 0, EPI_SD_G1IK = 256, EPI_SD_G1JI = 512,
               EPI_SD_T1I = 576, EPI_SD_T1J = 584, EPI_SD_DJ = 592,
               EPI_SD_G2JK = 600, EPI_SD_G2IK = 856, EPI_SD_G2JI = 1112,
               EPI_SD_F1I = 1176, EPI_SD_F1J = 1184, EPI_SD_SIZE = 1192;
+// The same-spin epilogue's: g1 of (j,k), (i,k), (j,i) as [b][c], then as
+// [b][a], t1[i,j,k][b] and d[j][b]; the f_ov half follows.
+constexpr int EPI_SA_BC = 0, EPI_SA_BA = 768, EPI_SA_T1 = 960,
+              EPI_SA_DJ = 984, EPI_SA_F = 992, EPI_SA_SIZE = 2 * EPI_SA_F;
 static_assert(EPI_THREADS == EPI_B * EPI_C && EPI_B * EPI_C == 256 &&
                   EPI_A * EPI_B == 64 && EPI_A == 8 && EPI_B == 8,
               "one staged (b, c) per thread; offsets above");
-
-__device__ __forceinline__ int64_t pairidx(int p, int q) {
-  return (int64_t)p * (p - 1) / 2 + q;
-}
 
 __device__ __forceinline__ int pair32(int p, int q) {
   return p * (p - 1) / 2 + q;
@@ -69,10 +83,52 @@ __device__ double block_sum(double x) {
 
 // ---------------------------------------------------------------- aaa ----
 
-// Thread layout of both epilogues: warp w handles a = a0 + w, lane l handles
-// c = c0 + l, and each thread walks the tile's 8 values of b (unrolled,
-// branch-free with clamped indices and a validity mask, so the loads of
-// several b are in flight together).
+// Four doubles of a contraction output (32-byte aligned; written by an
+// earlier launch).
+__device__ __forceinline__ void load4(const double *p, double *v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+      : "l"(p));
+}
+
+// v[k] += row[p0 + k], k < 8, by aligned loads of four: p0 % 4 is the same
+// for the whole warp.  Loads past the row (ld, a multiple of 4) are moved
+// back into it; their elements are not needed.
+__device__ __forceinline__ void add8_at(const double *row, int p0, int ld,
+                                        double (&v)[8]) {
+  double q[12];
+  const int b = p0 & ~3, last = ld - 4;
+  load4(row + min(b, last), q);
+  load4(row + min(b + 4, last), q + 4);
+  switch (p0 & 3) {
+    case 0:
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += q[k];
+      return;
+    case 1:
+      load4(row + min(b + 8, last), q + 8);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += q[k + 1];
+      return;
+    case 2:
+      load4(row + min(b + 8, last), q + 8);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += q[k + 2];
+      return;
+    default:
+      load4(row + min(b + 8, last), q + 8);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += q[k + 3];
+      return;
+  }
+}
+
+// row[x0 .. x0 + 7] of a row of ld doubles (x0, ld multiples of 4).
+__device__ __forceinline__ void load8(const double *row, int x0, int ld,
+                                      double (&v)[8]) {
+  load4(row + x0, v);
+  load4(row + (x0 + 4 < ld ? x0 + 4 : x0), v + 4);
+}
 
 // 8-byte asynchronous global -> shared copy; ok == false writes 0.0 (the
 // source is not read: src-size 0 zero-fills the destination).
@@ -82,6 +138,35 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src,
       "cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)),
       "l"(src), "r"(ok ? 8 : 0)
       : "memory");
+}
+
+// The same for 16 bytes (both addresses 16-byte aligned).
+__device__ __forceinline__ void cp_async16(double *dst, const double *src,
+                                           bool ok) {
+  asm volatile(
+      "cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(ok ? 16 : 0)
+      : "memory");
+}
+
+// Staged runs of a packed pair row: [row][pair of doubles][c].
+__device__ __forceinline__ int pairs_at(int row, int x, int c) {
+  return ((row * 5 + (x >> 1)) * EPI_C + c) * 2 + (x & 1);
+}
+
+// The five pairs of base[c * ld + (p0 & ~1) ..] for the tile's 32 c.
+__device__ __forceinline__ void stage_pairs(double *dst, const double *base,
+                                            int64_t ld, int p0, int c0, int nc,
+                                            bool ok) {
+  const int row = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ok = ok && c0 + lane < nc;
+  const double *src = base + (ok ? (c0 + lane) * ld : 0);
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int x = (p0 & ~1) + 2 * q;
+    const bool in = ok && x < ld;
+    cp_async16(dst + pairs_at(row, 2 * q, lane), src + (in ? x : 0), in);
+  }
 }
 
 __device__ __forceinline__ void cp_async_wait_all() {
@@ -118,15 +203,12 @@ __device__ __forceinline__ void load_args(EpiArgs &dst, const EpiArgs *src) {
 }
 
 template <bool FT, bool LOOP, bool HASF>
-__global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
+__global__ void __launch_bounds__(EPI_THREADS, epi_minb(FT))
     epi_aaa_kernel(const EpiList *__restrict__ list,
                    const EpiItem *__restrict__ items) {
-  extern __shared__ double sm[];
+  extern __shared__ double sm[];   // EPI_SA_*, then (T): T[c][ab] runs
   __shared__ EpiArgs p;
-  constexpr int S = EPI_A * EPI_B * EPI_CS;
-  constexpr int NIT = EPI_A * EPI_C * EPI_B / EPI_THREADS;
-  // s3[a_][b_][c_] = T[c][pair(a,b)]  (the R copy follows for (fT))
-  double *s3 = sm;
+  double *s3 = sm + EPI_SA_SIZE;
   // LOOP: a fixed grid striding over the flat tiles of all items; else one
   // CTA per (tile, item) of a 2-D grid
   int blk = blockIdx.x;
@@ -157,41 +239,65 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   const double *base = item.ws;
   const double *T = base + p.offL[0];
   const double *R = FT ? base + p.offR[0] : nullptr;
-  const int64_t ld = p.ld[0];
-  const int ldi = (int)ld;
-
-  // stage T[c][pair(a,b)] asynchronously; its wait comes after the loads
-  // of the per-thread operands below, so both latencies overlap
-#pragma unroll
-  for (int it = 0; it < NIT; ++it) {
-    const int e = threadIdx.x + it * EPI_THREADS;
-    const int a_ = e / (EPI_C * EPI_B), c_ = (e / EPI_B) % EPI_C,
-              b_ = e % EPI_B;
-    const int a = a0 + a_, b = b0 + b_, c = c0 + c_;
-    const bool ok = a < v && b < a && c < b;
-    const int64_t off = ok ? (int64_t)c * ld + pairidx(a, b) : 0;
-    const int idx = (a_ * EPI_B + b_) * EPI_CS + c_;
-    cp_async8(&s3[idx], T + off, ok);
-    if (FT) cp_async8(&s3[S + idx], R + off, ok);
-  }
+  const int ldi = (int)p.ld[0];
 
   const int a_ = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + a_, c = c0 + lane;
   const int ac = a < v ? a : v - 1;       // clamped indices for addressing
   const int cc = c < v ? c : v - 1;
-  // disconnected term (src/pt.c:162-175): the parts that depend on (a, c)
+  if (!FT)
+    stage_pairs(s3, T, ldi, pair32(ac, b0), c0, v, a < v);
+  // disconnected term (src/pt.c:162-175)
   const int64_t sl1 = (int64_t)v * p.g1_ld_aa, sl2 = (int64_t)v * p.g2_ld_aa;
-  const double *g1jk = p.g1_aa + ((int64_t)j * o + k) * sl1;
-  const double *g1ik = p.g1_aa + ((int64_t)i * o + k) * sl1;
-  const double *g1ji = p.g1_aa + ((int64_t)j * o + i) * sl1;
-  const double *g2jk = p.g2_aa + ((int64_t)j * o + k) * sl2;
-  const double *g2ik = p.g2_aa + ((int64_t)i * o + k) * sl2;
-  const double *g2ji = p.g2_aa + ((int64_t)j * o + i) * sl2;
   const double *u1 = p.ov1_a, *u2 = p.ov2_a;
+  // its parts that vary with b are the same for every warp: staged once
+  // (zero outside the space; those elements are masked)
+  {
+    const int t = threadIdx.x;
+    const int bt = b0 + (t >> 5), ct = c0 + (t & 31);
+    const bool okbc = bt < v && ct < v;
+#pragma unroll
+    for (int h = 0; h < (HASF ? 2 : 1); ++h) {
+      if (h && !has_f) break;
+      const int64_t sl = h ? sl2 : sl1;
+      const int ld = h ? g2l : g1l;
+      const double *g = h ? p.g2_aa : p.g1_aa;
+      const double *gs[3] = {g + ((int64_t)j * o + k) * sl,
+                             g + ((int64_t)i * o + k) * sl,
+                             g + ((int64_t)j * o + i) * sl};
+      double *s = sm + h * EPI_SA_F;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        cp_async8(&s[EPI_SA_BC + 256 * q + t], gs[q] + (okbc ? bt * ld + ct : 0),
+                  okbc);
+      if (t < EPI_B * EPI_A) {
+        const int bb = b0 + (t >> 3), aa = a0 + (t & 7);
+        const bool ok = bb < v && aa < v;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          cp_async8(&s[EPI_SA_BA + 64 * q + t], gs[q] + (ok ? bb * ld + aa : 0),
+                    ok);
+      } else if (t < EPI_B * EPI_A + 3 * EPI_B) {
+        const int q = (t - EPI_B * EPI_A) >> 3, bb = b0 + (t & 7);
+        const int occ = q == 0 ? i : q == 1 ? j : k;
+        cp_async8(&s[EPI_SA_T1 + (t - EPI_B * EPI_A)],
+                  (h ? u2 : u1) + (bb < v ? occ * v + bb : 0), bb < v);
+      } else if (h == 0 && t < EPI_B * EPI_A + 4 * EPI_B) {
+        const int bb = b0 + (t & 7);
+        cp_async8(&s[EPI_SA_DJ + (t & 7)], p.d_a + (bb < v ? j * v + bb : 0),
+                  bb < v);
+      }
+    }
+  }
   const int64_t ac1 = (int64_t)ac * p.g1_ld_aa + cc,
                 ac2 = (int64_t)ac * p.g2_ld_aa + cc;
-  const double A1jk = g1jk[ac1], A1ik = g1ik[ac1], A1ji = g1ji[ac1];
-  const double A2jk = g2jk[ac2], A2ik = g2ik[ac2], A2ji = g2ji[ac2];
+  const double *g1 = p.g1_aa, *g2 = p.g2_aa;
+  const int64_t sjk = (int64_t)j * o + k, sik = (int64_t)i * o + k,
+                sji = (int64_t)j * o + i;
+  const double A1jk = g1[sjk * sl1 + ac1], A1ik = g1[sik * sl1 + ac1],
+               A1ji = g1[sji * sl1 + ac1];
+  const double A2jk = g2[sjk * sl2 + ac2], A2ik = g2[sik * sl2 + ac2],
+               A2ji = g2[sji * sl2 + ac2];
   const double t1ia = u1[i * v + ac], t1ja = u1[j * v + ac],
                t1ka = u1[k * v + ac];
   const double t1ic = u1[i * v + cc], t1jc = u1[j * v + cc],
@@ -201,39 +307,52 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   const double f_ic = u2[i * v + cc], f_jc = u2[j * v + cc],
                f_kc = u2[k * v + cc];
   const double dia = p.d_a[i * v + ac], dkc = p.d_a[k * v + cc];
+  // W (and R) of the thread's 8 b; the pair index needs c < b (else any
+  // element of the row: those are masked)
+  double w8[EPI_B], r8[EPI_B];
+#pragma unroll
+  for (int side = 0; side < (FT ? 2 : 1); ++side) {
+    const double *X = side ? R : T;
+    double(&w)[EPI_B] = side ? r8 : w8;
+#pragma unroll
+    for (int b_ = 0; b_ < EPI_B; ++b_) {
+      const int b = b0 + b_;
+      const int bc = b < v ? b : v - 1;
+      const int cb = c < b && b < a && a < v ? c : 0;
+      // offsets < 2^31 (checked by the plan)
+      w[b_] = X[ac * ldi + pair32(bc, cb)] - X[bc * ldi + pair32(ac, cb)];
+    }
+    if (FT) add8_at(X + (int64_t)cc * ldi, pair32(ac, b0), ldi, w);
+  }
   cp_async_wait_all();
   __syncthreads();
 
-  // one b at a time: the element's energy is added as soon as its operands
-  // are in (arrays of all 8 b values spilled registers); the loop is
-  // unrolled so the loads of later b overlap the arithmetic of earlier ones
   double e = 0.0;
 #pragma unroll
   for (int b_ = 0; b_ < EPI_B; ++b_) {
     const int b = b0 + b_;
     const bool ok = a < v && b < a && c < b;
-    const int bc = b < v ? b : v - 1;
-    const int cb = ok ? c : 0;               // pair index needs c < b
-    const int t1 = ac * ldi + pair32(bc, cb);   // < 2^31 (plan check)
-    const int t2 = bc * ldi + pair32(ac, cb);
-    const int is = (a_ * EPI_B + b_) * EPI_CS + lane;
-    const double w = T[t1] - T[t2] + s3[is];
-    const double rr = FT ? R[t1] - R[t2] + s3[S + is] : w;
-    const int bc1 = bc * g1l + cc, bc2 = bc * g2l + cc;
-    const int ba1 = bc * g1l + ac, ba2 = bc * g2l + ac;
+    const double w =
+        FT ? w8[b_]
+           : w8[b_] + s3[pairs_at(a_, b_ + (pair32(ac, b0) & 1), lane)];
+    const double rr = FT ? r8[b_] : w;
+    const double *bc = sm + EPI_SA_BC + b_ * EPI_C + lane;
+    const double *ba = sm + EPI_SA_BA + b_ * EPI_A + a_;
+    const double *tb = sm + EPI_SA_T1 + b_;
     // the 9-term sums of src/pt.c:166-174 for (t1, i_oovv) and (f_ov, t2);
     // the second is skipped when f_ov is zero (its terms would all be 0)
-    double x =
-        t1ia * g1jk[bc1] - t1ja * g1ik[bc1] - t1ka * g1ji[bc1] -
-        u1[i * v + bc] * A1jk + u1[j * v + bc] * A1ik +
-        u1[k * v + bc] * A1ji - t1ic * g1jk[ba1] + t1jc * g1ik[ba1] +
-        t1kc * g1ji[ba1];
-    if (has_f)
-      x += f_ia * g2jk[bc2] - f_ja * g2ik[bc2] - f_ka * g2ji[bc2] -
-           u2[i * v + bc] * A2jk + u2[j * v + bc] * A2ik +
-           u2[k * v + bc] * A2ji - f_ic * g2jk[ba2] + f_jc * g2ik[ba2] +
-           f_kc * g2ji[ba2];
-    const double dd = (dia + p.d_a[j * v + bc]) + dkc;
+    double x = t1ia * bc[0] - t1ja * bc[256] - t1ka * bc[512] - tb[0] * A1jk +
+               tb[8] * A1ik + tb[16] * A1ji - t1ic * ba[0] + t1jc * ba[64] +
+               t1kc * ba[128];
+    if (has_f) {
+      bc += EPI_SA_F;
+      ba += EPI_SA_F;
+      tb += EPI_SA_F;
+      x += f_ia * bc[0] - f_ja * bc[256] - f_ka * bc[512] - tb[0] * A2jk +
+           tb[8] * A2ik + tb[16] * A2ji - f_ic * ba[0] + f_jc * ba[64] +
+           f_kc * ba[128];
+    }
+    const double dd = (dia + sm[EPI_SA_DJ + b_]) + dkc;
     if (ok) e += (w - x) * rr * recip_nr(dd);
   }
   const double s = block_sum(e);
@@ -248,16 +367,16 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
 // ---------------------------------------------------------------- aab ----
 
 template <bool FT, bool LOOP, bool HASF>
-__global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
+__global__ void __launch_bounds__(EPI_THREADS, epi_minb(FT))
     epi_aab_kernel(const EpiList *__restrict__ list,
                    const EpiItem *__restrict__ items) {
   extern __shared__ double sm[];
   __shared__ EpiArgs p;
-  constexpr int S = EPI_A * EPI_B * EPI_CS;
-  constexpr int NIT = EPI_A * EPI_C * EPI_B / EPI_THREADS;
-  // sx[a_][b_][c_] = U2[a][c][b];  sy[b_][a_][c_] = U2[b][c][a];
-  // sp[a_][b_][c_] = P[c][pair(a,b)]   (R copies follow for (fT))
-  double *sx = sm, *sy = sm + S, *sp = sm + 2 * S;
+  constexpr int S = EPI_A * EPI_B * (FT ? EPI_C : EPI_CS);
+  // (T): sy[b_][a_][c_] = U2[b][c][a], sx[a_][b_][c_] = U2[a][c][b],
+  //      sp[a_][b_][c_] = P[c][pair(a,b)]
+  // (fT): sy, then its R copy
+  double *sy = sm, *sx = sm + S, *sp = sm + 2 * S;
   // LOOP: a fixed grid striding over the flat tiles of all items; else one
   // CTA per (tile, item) of a 2-D grid
   int blk = blockIdx.x;
@@ -293,8 +412,8 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   const int i = item.i, j = item.j, k = item.k;
   const int oa = p.oa, va = p.va, ob = p.ob, vb = p.vb;
   const double *base = item.ws;
-  const int64_t ld2 = p.ld[1], ldp = p.ld[2];
-  const int64_t r2 = p.rowU2;
+  const int64_t ld2 = p.ld[1];
+  const int ldp = (int)p.ld[2], r2 = (int)p.rowU2;
   // 32-bit strides for the per-element loop (the plan keeps a triple's
   // arrays and the i_oovv / amplitude slices under 2^31 elements)
   const int ld1 = (int)p.ld[0], r1 = (int)p.rowU1;
@@ -302,40 +421,32 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   const int g1laa = (int)p.g1_ld_aa, g2laa = (int)p.g2_ld_aa;
   const bool has_f = HASF && p.has_f != 0;   // HASF false: f_ov is zero
 
-  // stage U2 (both orientations) and P asynchronously; the wait comes after
-  // the per-thread operand loads below
-#pragma unroll
-  for (int side = 0; side < (FT ? 2 : 1); ++side) {
-    const int64_t *off = side ? p.offR : p.offL;
-    const double *U2 = base + off[1];
-    const double *P = base + off[2];
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int e = threadIdx.x + it * EPI_THREADS;
-      const int u = e / (EPI_C * EPI_B), c_ = (e / EPI_B) % EPI_C,
-                w = e % EPI_B;
-      const int c = c0 + c_;
-      const bool cok = c < vb;
-      const int idx = side * 3 * S + (u * EPI_B + w) * EPI_CS + c_;
-      const int ax = a0 + u, bx = b0 + w;     // x: U2[a][c][b]
-      const bool okx = cok && ax < va && bx < va;
-      cp_async8(&sx[idx], U2 + (okx ? (int64_t)ax * ld2 + c * r2 + bx : 0),
-                okx);
-      const int by = b0 + u, ay = a0 + w;     // y: U2[b][c][a]
-      const bool oky = cok && ay < va && by < va;
-      cp_async8(&sy[idx], U2 + (oky ? (int64_t)by * ld2 + c * r2 + ay : 0),
-                oky);
-      const bool okp = cok && ax < va && bx < ax;   // p: P[c][pair(a,b)]
-      cp_async8(&sp[idx],
-                P + (okp ? (int64_t)c * ldp + pairidx(ax, bx) : 0), okp);
-    }
-  }
-
   const int a_ = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + a_, c = c0 + lane;
   const int ac = a < va ? a : va - 1, cc = c < vb ? c : vb - 1;
-  const double *U1 = base + p.offL[0];
-  const double *U1r = FT ? base + p.offR[0] : nullptr;
+  if (!FT) {
+    // thread: one (c, w) of every row u, w the index within the run
+    const int w = threadIdx.x & 7, cs = threadIdx.x >> 3, cg = c0 + cs;
+    const bool cok = cg < vb;
+    const int ax0 = a0, bx = b0 + w, ay = a0 + w;
+    const double *px = base + p.offL[1] + (int64_t)a0 * ld2 + cg * r2 + bx;
+    const double *py = base + p.offL[1] + (int64_t)b0 * ld2 + cg * r2 + ay;
+    const double *pp = base + p.offL[2] + (int64_t)cg * ldp + pair32(a0, bx);
+    const bool xok = cok && bx < va, yok = cok && ay < va;
+#pragma unroll
+    for (int u = 0; u < EPI_A; ++u) {
+      const int ax = ax0 + u;
+      const int idx = (u * EPI_B + w) * EPI_CS + cs;
+      const bool okx = xok && ax < va, oky = yok && b0 + u < va;
+      const bool okp = okx && bx < ax;
+      cp_async8(&sx[idx], okx ? px : base, okx);
+      cp_async8(&sy[idx], oky ? py : base, oky);
+      cp_async8(&sp[idx], okp ? pp : base, okp);
+      px += ld2;
+      py += ld2;
+      pp += ax;   // pair(a + 1, b) = pair(a, b) + a
+    }
+  }
   // disconnected-term slices (src/pt.c:433-442)
   const double *g1jk = p.g1_ab + ((int64_t)j * ob + k) * va * p.g1_ld_ab;
   const double *g1ik = p.g1_ab + ((int64_t)i * ob + k) * va * p.g1_ld_ab;
@@ -349,7 +460,7 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   // every warp (a) of the tile: staged once into shared memory (zero where
   // b or c is outside the space; those elements are masked) instead of
   // loaded by each warp in the b loop.
-  double *sd = sm + (FT ? 6 : 3) * S;
+  double *sd = sm + (FT ? 2 : 3) * S;
   {
     const int t = threadIdx.x;   // one (b, c) per thread
     const int bt = b0 + (t >> 5), ct = c0 + (t & 31);
@@ -390,33 +501,47 @@ __global__ void __launch_bounds__(EPI_THREADS, EPI_MINB)
   const double f_ia = u2[i * va + ac], f_ja = u2[j * va + ac];
   const double o1k = p.ov1_b[k * vb + cc], o2k = p.ov2_b[k * vb + cc];
   const double dia = p.d_a[i * va + ac], dkc = p.d_b[k * vb + cc];
-  // U1 in both orientations, loaded before the wait for the staged
-  // operands so that the two sets of loads are in flight together (the
-  // wait is a memory barrier for the compiler)
-  double xu[EPI_B];
+  // U1 in both orientations, and for (fT) all of W and R but U2[b][c][a],
+  // which this warp reads for b = b0 + a_ and stages for the others
+  double w8[EPI_B], r8[EPI_B];
 #pragma unroll
-  for (int b_ = 0; b_ < EPI_B; ++b_) {
-    const int bc = b0 + b_ < va ? b0 + b_ : va - 1;
-    xu[b_] = U1[ac * ld1 + bc * r1 + cc] - U1[bc * ld1 + ac * r1 + cc];
-  }   // offsets < 2^31 (checked by the plan)
+  for (int side = 0; side < (FT ? 2 : 1); ++side) {
+    const int64_t *off = side ? p.offR : p.offL;
+    const double *U1 = base + off[0], *U2 = base + off[1], *P = base + off[2];
+    double(&w)[EPI_B] = side ? r8 : w8;
+    if (FT) {
+      const int by = b0 + a_ < va ? b0 + a_ : va - 1;
+      double y[EPI_A];
+      load8(U2 + (int64_t)by * ld2 + cc * r2, a0, r2, y);
+      load8(U2 + (int64_t)ac * ld2 + cc * r2, b0, r2, w);
+#pragma unroll
+      for (int x = 0; x < EPI_A; ++x)
+        sy[side * S + (a_ * EPI_A + x) * EPI_C + lane] = y[x];
+    }
+#pragma unroll
+    for (int b_ = 0; b_ < EPI_B; ++b_) {   // offsets < 2^31 (plan check)
+      const int bc = b0 + b_ < va ? b0 + b_ : va - 1;
+      const double u =
+          U1[ac * ld1 + bc * r1 + cc] - U1[bc * ld1 + ac * r1 + cc];
+      w[b_] = FT ? w[b_] + u : u;
+    }
+    if (FT) add8_at(P + (int64_t)cc * ldp, pair32(ac, b0), ldp, w);
+  }
   cp_async_wait_all();
   __syncthreads();
 
-  // one b at a time (see the same-spin kernel)
   double e = 0.0;
 #pragma unroll
   for (int b_ = 0; b_ < EPI_B; ++b_) {
     const int b = b0 + b_;
     const bool ok = a < va && b < a && c < vb;
-    const int bc = b < va ? b : va - 1;
-    const int u_ab = ac * ld1 + bc * r1 + cc;
-    const int u_ba = bc * ld1 + ac * r1 + cc;
-    const int ix = (a_ * EPI_B + b_) * EPI_CS + lane;
-    const int iy = (b_ * EPI_A + a_) * EPI_CS + lane;
-    const double w = xu[b_] + sx[ix] - sy[iy] + sp[ix];
-    const double rr = FT ? U1r[u_ab] + sx[3 * S + ix] - U1r[u_ba] -
-                               sy[3 * S + iy] + sp[3 * S + ix]
-                         : w;
+    constexpr int CS = FT ? EPI_C : EPI_CS;
+    const int ix = (a_ * EPI_B + b_) * CS + lane;
+    const int iy = (b_ * EPI_A + a_) * CS + lane;
+    const double w =
+        FT ? w8[b_] - sy[iy]
+           : w8[b_] + sx[ix] - sy[iy] + sp[ix];
+    const double rr = FT ? r8[b_] - sy[S + iy] : w;
     const int bcl = b_ * EPI_C + lane, ba = b_ * EPI_A + a_;
     double x = t1ia * sd[EPI_SD_G1JK + bcl] - sd[EPI_SD_T1I + b_] * A1jk -
                t1ja * sd[EPI_SD_G1IK + bcl] + sd[EPI_SD_T1J + b_] * A1ik +
@@ -475,9 +600,11 @@ cudaError_t launch_epi(K kern, const EpiList *d_list, const EpiItem *d_items,
 }  // namespace
 
 size_t epi_smem_bytes(bool aab, bool ft) {
-  const size_t s = (size_t)EPI_A * EPI_B * EPI_CS * sizeof(double);
-  return (aab ? 3 : 1) * (ft ? 2 : 1) * s +
-         (aab ? EPI_SD_SIZE * sizeof(double) : 0);
+  const size_t ab = (size_t)EPI_A * EPI_B;
+  const size_t pairs = (size_t)EPI_A * 10 * EPI_C;   // runs of a packed row
+  return (aab ? (ft ? 2 * ab * EPI_C : 3 * ab * EPI_CS) + EPI_SD_SIZE
+              : EPI_SA_SIZE + (ft ? 0 : pairs)) *
+         sizeof(double);
 }
 
 int epi_blocks_per_sm(bool aab, bool ft) {
