@@ -156,19 +156,16 @@ cudaError_t gemm_tc_launch(const GemmJob *d_jobs, GemmList *d_list,
 // ---- emulated FP64 (tcgen05 kind::i8, gemm_i8.cu) ---------------------------
 //
 // S digit planes per operand, the products with p + q <= S - 1 (0-based)
-// into S INT32 accumulators of bn columns.  The digit planes are a
-// coordinate of one map per operand: A maps [2S][P][Q][kpi/32][R][32] hold
-// the digits then their negatives, B maps [S][P][kpi/32][N][32]; 32-byte K
-// chunks of 128 (A) or bn (B) rows are contiguous, read as one TMA box each
-// and swizzled to 32 bytes.  An A segment's (Q, P) coordinates are merged
-// into a_q = a_p * Q + a_q.
+// into S INT32 accumulators of bn columns; a tile is bn rows by 128 columns of
+// C.  The digit planes are a coordinate of one map per operand: A maps
+// [2S][P][Q][kpi/64][R][64] hold the digits then their negatives, B maps
+// [S][P][kpi/64][N][64]; 64-byte K chunks of bn (A) or 128 (B) rows are
+// contiguous, read as one TMA box each and swizzled to 64 bytes.  An A
+// segment's (Q, P) coordinates are merged into a_q = a_p * Q + a_q.
 struct I8Tile {
-  int bn;     // tile columns (multiple of 16, S * bn <= 512)
+  int bn;     // rows of C per tile (multiple of 16, S * bn <= 512)
   int kc;     // K bytes per pipeline stage (I8_KCHUNK: two MMA K steps)
-  int pair;   // 1: a CTA pair (two SMs) computes a 256 x bn tile, each CTA
-              // loading its 128 rows of A and half of the bn columns of B
-  int ts;     // 1: the MMAs read A from TMEM (copied there once per plane
-              // and K step) instead of re-reading it from shared memory
+  int cost;   // relative time of a full tile's row
 };
 // Digit planes are stored in K chunks of I8_KCHUNK bytes (64: one 64-byte
 // swizzled row per TMA box row; a box of R rows is one contiguous block).

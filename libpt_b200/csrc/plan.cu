@@ -120,10 +120,6 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
     const double v = std::atof(t);
     if (v > 0) p->emu_tol = v;
   }
-  {
-    const I8Tile *t = nullptr;
-    if (i8_tiles(slices, &t) > 0) p->i8tile = t[0];   // widest tile
-  }
   p->st = st;
   p->factor = unr ? 1.0 : 2.0;   // src/pt.c:478, 534, 971, 1049
   p->arena = static_cast<char *>(arena);

@@ -175,7 +175,7 @@ struct libpt_plan {
   int dbits = 7;                        // digit base bits of the planes (7, 8)
   bool slices_auto = false;             // choose slices for emu_tol
   double emu_tol = 1e-6;                // |dE| target of the choice (Eh)
-  ptb::I8Tile i8tile{64, ptb::I8_KCHUNK, 0, 0};   // emulated FP64 tile variant
+  ptb::I8Tile i8tile{64, ptb::I8_KCHUNK, 100};   // emulated FP64 tile variant
   std::vector<std::pair<std::pair<const double *, int>, signed char *>> i8planes;
   std::vector<ptb::Family> fams;
   // kernel timing (libpt_plan_timing): events around each round's GEMMs
@@ -214,14 +214,14 @@ size_t plan_footprint(int kind, size_t oa, size_t va, size_t ob, size_t vb,
 int tc_map_a(CUtensorMap *m, const float *p, int64_t K, int64_t R, int64_t Q,
              int64_t P);
 int tc_map_b(CUtensorMap *m, const float *p, int64_t K, int64_t N, int64_t P);
-// INT8 digit-plane views: A planes [2S][P][Q][kpi/32][R][32] as
-// (32, R, kpi/32, Q*P, 2S), B planes [S][P][kpi/32][N][32] as
-// (32, N, kpi/32, P, S); kpi = i8_kpad(K).  Boxes of 32 bytes x 128 (A) or
-// bn (B) rows, swizzled to 32 bytes.
+// INT8 digit-plane views: A planes [2S][P][Q][kpi/64][R][64] as
+// (64, R, kpi/64, Q*P, 2S), B planes [S][P][kpi/64][N][64] as
+// (64, N, kpi/64, P, S); kpi = i8_kpad(K).  Boxes of 64 bytes x bn (A) or
+// 128 (B) rows, swizzled to 64 bytes.
 int i8_map_a(CUtensorMap *m, const signed char *p, int64_t K, int64_t R,
-             int64_t Q, int64_t P, int S);
+             int64_t Q, int64_t P, int S, int bn);
 int i8_map_b(CUtensorMap *m, const signed char *p, int64_t K, int64_t N,
-             int64_t P, int S, int bn);
+             int64_t P, int S);
 // DMMA views of padded FP64 blocks: A [P][Q][R][pad4(K)], B [P][K][Nld].
 int dmma_map_a(CUtensorMap *m, const double *p, int64_t K, int64_t R,
                int64_t Q, int64_t P, int bm);

@@ -98,11 +98,9 @@ int i8_encode(libpt_plan *p, SpinCase &c) {
     const int r =
         d.role == 0
             ? i8_map_a(&c.tcmaps.m[i], c.i8pl[i], d.K, d.R, d.Q, d.P,
-                       p->slices_store)
+                       p->slices_store, p->i8tile.bn)
             : i8_map_b(&c.tcmaps.m[i], c.i8pl[i], d.K, d.N, d.P,
-                       p->slices_store,
-                       // a CTA of a pair tile loads half of its columns
-                       p->i8tile.pair ? p->i8tile.bn / 2 : p->i8tile.bn);
+                       p->slices_store);
     if (r) return r;
   }
   return LIBPT_OK;
@@ -150,6 +148,31 @@ int i8_planes(libpt_plan *p, SpinCase &c) {
   return LIBPT_OK;
 }
 
+// The INT8 tile variant a plan starts from: the least modelled time of its
+// jobs, whose rows are padded to whole tiles (v = 143, S = 5: two tiles of 80
+// rows, not two of 96).
+I8Tile i8_default_tile(const libpt_plan *p, int S) {
+  const I8Tile *t = nullptr;
+  const int n = i8_tiles(S, &t);
+  I8Tile best = t[0];
+  double least = -1.0;
+  for (int x = 0; x < n; ++x) {
+    double w = 0.0;
+    for (const SpinCase &c : p->cases)
+      for (const JobT &j : c.jobs) {
+        double k = 0.0;
+        for (int s = 0; s < j.nseg; ++s) k += j.seg[s].k;
+        w += (double)c.count * j.N * k * ((j.M + t[x].bn - 1) / t[x].bn) *
+             t[x].bn * t[x].cost;
+      }
+    if (least < 0.0 || w < least) {
+      least = w;
+      best = t[x];
+    }
+  }
+  return best;
+}
+
 // Digit width of the INT8 planes.  Every accumulator (one digit-weight
 // diagonal: at most S digit products per unit of K, summed over a job's
 // segments) must stay below 2^31: S * 64^2 per unit of K for 7-bit digits,
@@ -174,11 +197,10 @@ int choose_digits(libpt_plan *p) {
     const int S = fits8(6) ? 6 : TC_S_MAX;
     p->dbits = S == 6 ? 8 : 7;
     p->slices = p->slices_store = S;
-    const I8Tile *t = nullptr;
-    if (i8_tiles(S, &t) > 0) p->i8tile = t[0];
   } else {
     p->dbits = fits8(p->slices_store) ? 8 : 7;
   }
+  p->i8tile = i8_default_tile(p, p->slices);
   if (p->dbits == 7 &&
       (double)kmax * 4096.0 * p->slices_store >= 2147483648.0) {
     set_error("emulated FP64: contraction too long for exact INT32 "
@@ -215,10 +237,8 @@ int choose_slices(libpt_plan *p) {
   const char *bound_env = std::getenv("LIBPT_EMU_BOUND");
   const bool worst = bound_env && std::strcmp(bound_env, "worst") == 0;
   auto apply = [&](int S) -> int {
-    const I8Tile *tiles = nullptr;
-    if (i8_tiles(S, &tiles) <= 0) return LIBPT_ERR_ARG;
     p->slices = S;
-    p->i8tile = tiles[0];
+    p->i8tile = i8_default_tile(p, S);
     for (SpinCase &c : p->cases)
       if (c.count)
         if (int r = i8_encode(p, c)) return r;

@@ -145,8 +145,8 @@ int plan_append(libpt_plan *p, const int64_t *ents, size_t n, PlanCursor &cur,
     const CUtensorMap *hmaps = p->precision == LIBPT_PREC_FP64 ? c.maps.m
                                                                : c.tcmaps.m;
     const int map0 = r.maps[grp].add(c.d_maps, hmaps, tc ? TC_MAX_MAPS : MAX_MAPS);
-    const int bn = tc ? TC_BN : i8 ? p->i8tile.bn : GEMM_BN;
-    const int bmr = tc ? TC_BM : i8 ? (p->i8tile.pair ? 2 : 1) * TC_BM : c.bm;
+    const int bn = tc ? TC_BN : i8 ? TC_BM : GEMM_BN;
+    const int bmr = tc ? TC_BM : i8 ? p->i8tile.bn : c.bm;
     for (const JobT &jt : c.jobs) {
       GemmJob g;
       memset(&g, 0, sizeof(g));

@@ -146,7 +146,7 @@ int autotune(libpt_plan *p) {
       if (!r) r = probe_ms(p, p->cases[big], ents, &ms);
       if (!r && tune_verbose())
         std::fprintf(stderr, "libpt autotune %s: INT8 tile %dx%d, K chunk %d B: %.3f ms\n",
-                     key.c_str(), (tiles[t].pair ? 2 : 1) * TC_BM, tiles[t].bn,
+                     key.c_str(), TC_BM, tiles[t].bn,
                      tiles[t].kc, ms);
       if (!r && (t == 0 || ms < best_ms)) {
         best = t;

@@ -107,11 +107,11 @@ int tc_encode(CUtensorMap *m, const float *p, int rank, const cuuint64_t *dims,
   return LIBPT_OK;
 }
 
-// Digit-plane views (see slice_a / slice_b): 32-byte K chunks of rows
-// stored contiguously, boxes of 32 bytes x 128 (A) or bn (B) rows swizzled
-// to 32 bytes.  A: (32, R, nK, Q*P, 2S); B: (32, N, nK, P, S).
+// Digit-plane views (see slice_a / slice_b): 64-byte K chunks of rows
+// stored contiguously, boxes of 64 bytes x bn (A) or 128 (B) rows swizzled
+// to 64 bytes.  A: (64, R, nK, Q*P, 2S); B: (64, N, nK, P, S).
 int i8_map_a(CUtensorMap *m, const signed char *p, int64_t K, int64_t R,
-             int64_t Q, int64_t P, int S) {
+             int64_t Q, int64_t P, int S, int bn) {
   if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
   EncodeTiledFn enc = encode_fn();
   if (!enc) {
@@ -124,7 +124,7 @@ int i8_map_a(CUtensorMap *m, const signed char *p, int64_t K, int64_t R,
                         (cuuint64_t)(2 * S)};
   cuuint64_t str[4] = {W, (cuuint64_t)(R * W), (cuuint64_t)(R * kpi),
                        (cuuint64_t)(npq * R * kpi)};
-  cuuint32_t box[5] = {W, (cuuint32_t)TC_BM, 1, 1, 1};
+  cuuint32_t box[5] = {W, (cuuint32_t)bn, 1, 1, 1};
   cuuint32_t es[5] = {1, 1, 1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)p, dims, str,
                    box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -139,7 +139,7 @@ int i8_map_a(CUtensorMap *m, const signed char *p, int64_t K, int64_t R,
 }
 
 int i8_map_b(CUtensorMap *m, const signed char *p, int64_t K, int64_t N,
-             int64_t P, int S, int bn) {
+             int64_t P, int S) {
   if (g_dry) return LIBPT_OK;   // sizing pass: no views needed
   EncodeTiledFn enc = encode_fn();
   if (!enc) {
@@ -152,7 +152,7 @@ int i8_map_b(CUtensorMap *m, const signed char *p, int64_t K, int64_t N,
                         (cuuint64_t)S};
   cuuint64_t str[4] = {W, (cuuint64_t)(N * W), (cuuint64_t)(N * kpi),
                        (cuuint64_t)(P * N * kpi)};
-  cuuint32_t box[5] = {W, (cuuint32_t)bn, 1, 1, 1};
+  cuuint32_t box[5] = {W, (cuuint32_t)TC_BM, 1, 1, 1};
   cuuint32_t es[5] = {1, 1, 1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)p, dims, str,
                    box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
