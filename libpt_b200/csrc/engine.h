@@ -257,13 +257,16 @@ cudaError_t reduce_partials_launch(const RedList *d_list, int grid,
 // ---- closed-shell triples (epi_closed.cu, plan_closed.cu) --------------------
 
 constexpr int GEPI_T = 8;                  // index block of a group's tiles
-constexpr int GEPI_THREADS = 6 * GEPI_T * GEPI_T;
+constexpr int GEPI_THREADS = 3 * GEPI_T * GEPI_T;
 // Energies of groups {i < j < k}: items as for the epilogues above, args with
 // the three contraction outputs in offL / offR, ld[0] = v pad4(v), rowU1 =
 // pad4(v), tiles = blocks (X >= Y >= Z); partials [4][nblk]: the same-spin
 // triple, then the mixed-spin (ij;k), (ik;j), (jk;i).  grid = most tiles.
-cudaError_t epi_closed_launch(const EpiItem *d_items, bool ft, bool hasf,
-                              int grid, int nitems, cudaStream_t st);
+// pair: items (f, s, f) instead, outputs A1 and Z in offL / offR [0], [1],
+// partials [nblk]; pad_ != 0: the triple is (ij;j), not (ij;i).
+cudaError_t epi_closed_launch(const EpiItem *d_items, bool pair, bool ft,
+                              bool hasf, int grid, int nitems,
+                              cudaStream_t st);
 // Largest deviation (dst[0]) and magnitude (dst[1]), as bit patterns, of
 // same-spin matrices from the antisymmetrised mixed-spin ones; see
 // epi_closed.cu.

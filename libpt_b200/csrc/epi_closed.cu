@@ -12,6 +12,10 @@
 // over (u, g) = (t1, i_oovv) and (f_ov, t2), abab blocks:
 //   W(ij;k)[a,b;c] = V[a,b,c] - V[b,a,c]   (a at i, b at j, c at k), and so on
 //   W(ijk)[a,b,c]  = the six signed permutations.
+// A mixed-spin triple with a repeated index, (ij;i) or (ij;j), is a pair: V of
+// (f, s, f), f the repeated index, is symmetric in its outer virtuals,
+//   V[a,b,c] = A1[a][b][c] + A1[c][b][a] + Z[b][a][c] + Z[b][c][a]
+// from two contraction outputs, A1 of rows f and Z of rows s.
 #include <algorithm>
 
 #include "common.cuh"
@@ -27,6 +31,8 @@ static_assert(T == 8, "one lane per c, 8 a values per thread");
 // that reads along any of its indices meet few bank conflicts
 constexpr int S2 = T + 1, S1 = T * S2 + T + 1;
 constexpr int PB = T * S1;
+// one block pair of a staged g slice: rows of T + 1
+constexpr int GB = T * (T + 1);
 
 // Block order of (a, b, c) in each of the six permutations of the tile's
 // index blocks (0, 1, 2) = (X, Y, Z).
@@ -43,42 +49,66 @@ __device__ __forceinline__ void ld4(const double *p, double *v) {
                : "l"(p));
 }
 
-// v[8] = A1[a][b][c] + A2[b][a][c] + A3[c][b][a] for a = a0 .. a0+7 (b and c
-// inside the space; zero beyond it).  ldr = v pad4(v), v4 = pad4(v).
+// 8-byte asynchronous global -> shared copy; ok == false writes 0.0.
+__device__ __forceinline__ void cp_async8(double *dst, const double *src,
+                                          bool ok) {
+  asm volatile(
+      "cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(ok ? 8 : 0)
+      : "memory");
+}
+
+// out[8] = A1[a][b][c] + A2[b][a][c] + A3[c][b][a] for a = a0 .. a0+7; a pair
+// also adds A2[b][c][a] (its A3 is A1).  b and c are inside the space, rows
+// past it are read at its last row and never used.  ldr = v pad4(v), v4 =
+// pad4(v).
+template <bool PAIR>
 __device__ __forceinline__ void gather(const double *A1, const double *A2,
                                        const double *A3, int64_t ldr, int v,
                                        int v4, int a0, int b, int c,
                                        double (&out)[T]) {
   double x[T], y[T], z[T];
   const double *p1 = A1 + b * v4 + c, *p2 = A2 + b * ldr + c,
-               *p3 = A3 + c * ldr + b * v4 + a0;
+               *p3 = (PAIR ? A1 : A3) + c * ldr + b * v4 + a0,
+               *p4 = A2 + b * ldr + c * v4 + a0;
+  const int hi = a0 + 4 < v4 ? 4 : 0;   // a0 < v: the row holds a0 .. a0+3
 #pragma unroll
   for (int a = 0; a < T; ++a) {
-    const bool ok = a0 + a < v;
-    x[a] = ok ? __ldg(p1 + (a0 + a) * ldr) : 0.0;
-    y[a] = ok ? __ldg(p2 + (a0 + a) * v4) : 0.0;
-    z[a] = 0.0;
+    const int ac = min(a0 + a, v - 1);
+    x[a] = __ldg(p1 + ac * ldr);
+    y[a] = __ldg(p2 + ac * v4);
   }
-  ld4(p3, z);                          // a0 < v: the row holds these four
-  if (a0 + 4 < v4) ld4(p3 + 4, z + 4);
+  ld4(p3, z);
+  ld4(p3 + hi, z + 4);
 #pragma unroll
   for (int a = 0; a < T; ++a) out[a] = x[a] + y[a] + z[a];
+  if (PAIR) {
+    ld4(p4, z);
+    ld4(p4 + hi, z + 4);
+#pragma unroll
+    for (int a = 0; a < T; ++a) out[a] += z[a];
+  }
 }
 
-// Energies of one tile of one group: the unordered index sets {x >= y >= z}
-// with x, y, z in the tile's blocks X >= Y >= Z.  384 threads: phase 1, one
-// permutation of the blocks per 64 threads (a thread holds 8 a of one (b, c))
-// gathers V and V - X into shared memory, so every contraction output is read
-// once; phase 2, one index set per thread, adds the four triples' energies.
+// Energies of one tile of one group or pair: the unordered index sets
+// {x >= y >= z} with x, y, z in the tile's blocks X >= Y >= Z.  Phase 1: V (and
+// R) of every permutation of the blocks into shared memory, 64 threads a
+// permutation, a thread holding 8 a of one (b, c), so every contraction output
+// is read once; a pair's V is symmetric in its outer virtuals and needs three
+// of the six.  Phase 2: an index set at a time, a thread keeping its (y, z):
+// X of its permutations from the staged g slices, then the energies.
 //
-// Bound: HBM, 24 v^3 bytes of contraction outputs a group (48 for (fT)).
-// One pass for the four triples reads them once; the general epilogues would
-// read 8 (3 v^3 / 6 + 3 * 5 v^3 / 2) bytes for the same triples, 2.6 times
-// as many, and evaluate nine disconnected terms a set instead of six shorter
-// ones.
-template <bool FT, bool HASF>
-__global__ void __launch_bounds__(GEPI_THREADS, 2)
+// Bound: HBM, 24 v^3 bytes of contraction outputs a group (48 for (fT), 16 and
+// 32 a pair).  One pass for the four triples reads them once; the general
+// epilogues would read 8 (3 v^3 / 6 + 3 * 5 v^3 / 2) bytes for the same
+// triples, 2.6 times as many, and evaluate nine disconnected terms a set
+// instead of six shorter ones.  CTAs of 192 threads, four an SM, so that one's
+// loads run beside another's arithmetic (two of 384 that kept V - X and V in
+// shared memory: 2.7 TB/s, a quarter of the cycles at barriers).
+template <bool FT, bool HASF, bool PAIR>
+__global__ void __launch_bounds__(GEPI_THREADS, 4)
     epi_closed_kernel(const EpiItem *__restrict__ items) {
+  constexpr int NP = PAIR ? 3 : 6;
   extern __shared__ double sm[];
   __shared__ EpiArgs p;
   __shared__ double sd[3][3][T], su[3][3][T], sf[3][3][T];   // [occ][block][]
@@ -94,91 +124,72 @@ __global__ void __launch_bounds__(GEPI_THREADS, 2)
   }
   __syncthreads();
   const int4 tl = p.tiles[tile];
-  const int blk[3] = {tl.x, tl.y, tl.z};
   const int v = p.va, o = p.oa, v4 = (int)p.rowU1;
   const int64_t ldr = p.ld[0];
-  const int occ[3] = {item.i, item.j, item.k};
+  const int oi = item.i, oj = item.j, ok_ = item.k;
   const bool has_f = HASF && p.has_f != 0;
+  auto block = [&](int n) { return n == 0 ? tl.x : n == 1 ? tl.y : tl.z; };
+  double *sW = sm, *sR = sm + NP * PB, *sg = sm + (FT ? 2 : 1) * NP * PB;
+  // g_jk, g_ik, g_ij on the six ordered block pairs (of both halves with f)
+#pragma unroll
+  for (int it = 0; it < (HASF ? 12 : 6); ++it) {
+    if (it >= 6 && !has_f) break;
+    const int e = threadIdx.x + (it % 6) * GEPI_THREADS;
+    const int sl = (e >> 6) / 6, pq = (e >> 6) % 6;
+    int P, Q, rest;
+    perm_blocks(pq, P, Q, rest);
+    const int r = block(P) + ((e >> 3) & 7), c = block(Q) + (e & 7);
+    const bool in = r < v && c < v;
+    const int ld = (int)(it < 6 ? p.g1_ld_ab : p.g2_ld_ab);
+    const double *g = (it < 6 ? p.g1_ab : p.g2_ab) +
+                      ((int64_t)(sl == 0 ? oj : oi) * o + (sl == 2 ? oj : ok_)) *
+                          v * ld;
+    cp_async8(&sg[((it / 6) * 18 + sl * 6 + pq) * GB + ((e >> 3) & 7) * (T + 1) +
+                  (e & 7)],
+              g + (in ? r * ld + c : 0), in);
+  }
   if (threadIdx.x < 9 * T) {
     const int q = threadIdx.x / (3 * T), bl = (threadIdx.x / T) % 3,
               x = threadIdx.x % T;
-    const int q_ = q == 0 ? occ[0] : q == 1 ? occ[1] : occ[2];
-    const int n = (bl == 0 ? blk[0] : bl == 1 ? blk[1] : blk[2]) + x;
-    const bool ok = n < v;
-    sd[q][bl][x] = ok ? p.d_a[q_ * v + n] : 0.0;
-    su[q][bl][x] = ok ? p.ov1_a[q_ * v + n] : 0.0;
-    sf[q][bl][x] = ok && has_f ? p.ov2_a[q_ * v + n] : 0.0;
+    const int occ = q == 0 ? oi : q == 1 ? oj : ok_;
+    const int n = block(bl) + x;
+    const bool in = n < v;
+    sd[q][bl][x] = in ? p.d_a[occ * v + n] : 0.0;
+    su[q][bl][x] = in ? p.ov1_a[occ * v + n] : 0.0;
+    sf[q][bl][x] = in && has_f ? p.ov2_a[occ * v + n] : 0.0;
   }
-  __syncthreads();
-
-  double *sU = sm, *sW = sm + 6 * PB;   // V - X, and V (or R)
-  {
-    const int pm = threadIdx.x / (T * T), bl = (threadIdx.x / T) % T,
-              cl = threadIdx.x % T;
+  const int yl = (threadIdx.x / T) % T, zl = threadIdx.x % T;
+  // (perm_blocks' order of (P, Q) is that of (a, b): pairs 0..5 = (X,Y) (X,Z)
+  // (Y,X) (Y,Z) (Z,X) (Z,Y))
+#pragma unroll 1
+  for (int pm = threadIdx.x / (T * T); pm < NP; pm += GEPI_THREADS / (T * T)) {
     int ab, bb, cb;
     perm_blocks(pm, ab, bb, cb);
-    const int a0 = ab == 0 ? blk[0] : ab == 1 ? blk[1] : blk[2];
-    const int b = (bb == 0 ? blk[0] : bb == 1 ? blk[1] : blk[2]) + bl;
-    const int c = (cb == 0 ? blk[0] : cb == 1 ? blk[1] : blk[2]) + cl;
-    const bool ok = b < v && c < v;
-    double w[T], u[T];
-    if (ok) {
-      const double *base = item.ws;
-      gather(base + p.offL[0], base + p.offL[1], base + p.offL[2], ldr, v, v4,
-             a0, b, c, w);
-      // X over (t1, i_oovv), then (f_ov, t2)
-      double x[T];
-      {
-        const int ld = (int)p.g1_ld_ab;
-        const int64_t sl = (int64_t)v * ld;
-        const double *gjk = p.g1_ab + ((int64_t)occ[1] * o + occ[2]) * sl;
-        const double *gik = p.g1_ab + ((int64_t)occ[0] * o + occ[2]) * sl;
-        const double *gij = p.g1_ab + ((int64_t)occ[0] * o + occ[1]) * sl;
-        const double g0 = gjk[b * ld + c], ub = su[1][bb][bl],
-                     uc = su[2][cb][cl];
+    const int a0 = block(ab), b = min(block(bb) + yl, v - 1),
+              c = min(block(cb) + zl, v - 1);
+    const double *base = item.ws;
+    double w[T];
+    gather<PAIR>(base + p.offL[0], base + p.offL[1], base + p.offL[2], ldr, v,
+                 v4, a0, b, c, w);
 #pragma unroll
-        for (int a = 0; a < T; ++a) {
-          const int ac = a0 + a < v ? a0 + a : v - 1;
-          x[a] = su[0][ab][a] * g0 + ub * gik[ac * ld + c] +
-                 uc * gij[ac * ld + b];
-        }
-      }
-      if (has_f) {
-        const int ld = (int)p.g2_ld_ab;
-        const int64_t sl = (int64_t)v * ld;
-        const double *gjk = p.g2_ab + ((int64_t)occ[1] * o + occ[2]) * sl;
-        const double *gik = p.g2_ab + ((int64_t)occ[0] * o + occ[2]) * sl;
-        const double *gij = p.g2_ab + ((int64_t)occ[0] * o + occ[1]) * sl;
-        const double g0 = gjk[b * ld + c], ub = sf[1][bb][bl],
-                     uc = sf[2][cb][cl];
+    for (int a = 0; a < T; ++a) sW[pm * PB + a * S1 + yl * S2 + zl] = w[a];
+    if (FT) {
+      gather<PAIR>(base + p.offR[0], base + p.offR[1], base + p.offR[2], ldr,
+                   v, v4, a0, b, c, w);
 #pragma unroll
-        for (int a = 0; a < T; ++a) {
-          const int ac = a0 + a < v ? a0 + a : v - 1;
-          x[a] += sf[0][ab][a] * g0 + ub * gik[ac * ld + c] +
-                  uc * gij[ac * ld + b];
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < T; ++a) u[a] = w[a] - x[a];
-      if (FT)
-        gather(base + p.offR[0], base + p.offR[1], base + p.offR[2], ldr, v,
-               v4, a0, b, c, w);
-    } else {
-#pragma unroll
-      for (int a = 0; a < T; ++a) u[a] = w[a] = 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < T; ++a) {
-      sU[pm * PB + a * S1 + bl * S2 + cl] = u[a];
-      sW[pm * PB + a * S1 + bl * S2 + cl] = w[a];
+      for (int a = 0; a < T; ++a) sR[pm * PB + a * S1 + yl * S2 + zl] = w[a];
     }
   }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
   double e[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int s = threadIdx.x; s < T * T * T; s += GEPI_THREADS) {
-    const int xl = s / (T * T), yl = (s / T) % T, zl = s % T;
-    const int x = blk[0] + xl, y = blk[1] + yl, z = blk[2] + zl;
+  const int y = tl.y + yl, z = tl.z + zl;
+  const double diy = sd[0][1][yl], djy = sd[1][1][yl], dky = sd[2][1][yl];
+  const double diz = sd[0][2][zl], djz = sd[1][2][zl], dkz = sd[2][2][zl];
+#pragma unroll 1
+  for (int xl = threadIdx.x / (T * T); xl < T; xl += GEPI_THREADS / (T * T)) {
+    const int x = tl.x + xl;
     const bool xy = x > y, yz = y > z;
     // a set with a repeated index has one mixed-spin assignment, not three
     if (x >= v || y >= v || z >= v || x < y || y < z || !(xy || yz)) continue;
@@ -189,21 +200,51 @@ __global__ void __launch_bounds__(GEPI_THREADS, 2)
                        zl * S1 + xl * S2 + yl, zl * S1 + yl * S2 + xl};
     double u[6], w[6];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      u[q] = sU[q * PB + at[q]];
-      w[q] = sW[q * PB + at[q]];
+    for (int q = 0; q < NP; ++q) {
+      u[q] = sW[q * PB + at[q]];
+      w[q] = FT ? sR[q * PB + at[q]] : u[q];
     }
-    // 1 / (d_i + d_j + d_k), of each permutation that an energy uses
-    const double r0 =
-        recip_nr((sd[0][0][xl] + sd[1][1][yl]) + sd[2][2][zl]);
-    const double r1 =
-        recip_nr((sd[0][0][xl] + sd[1][2][zl]) + sd[2][1][yl]);
-    const double r2 =
-        recip_nr((sd[0][1][yl] + sd[1][0][xl]) + sd[2][2][zl]);
-    const double r3 =
-        recip_nr((sd[0][1][yl] + sd[1][2][zl]) + sd[2][0][xl]);
-    const double r4 =
-        recip_nr((sd[0][2][zl] + sd[1][0][xl]) + sd[2][1][yl]);
+    // X, subtracted from u: pairs 0..5 of a slice at the set's elements
+    const int gp[6] = {0 * GB + xl * (T + 1) + yl, 1 * GB + xl * (T + 1) + zl,
+                       2 * GB + yl * (T + 1) + xl, 3 * GB + yl * (T + 1) + zl,
+                       4 * GB + zl * (T + 1) + xl, 5 * GB + zl * (T + 1) + yl};
+#pragma unroll
+    for (int h = 0; h < (HASF ? 2 : 1); ++h) {
+      if (h && !has_f) break;
+      const double(*t)[3][T] = h ? sf : su;
+      const double *jk = sg + h * 18 * GB, *ik = jk + 6 * GB, *ij = ik + 6 * GB;
+      const double ix = t[0][0][xl], iy = t[0][1][yl], iz = t[0][2][zl];
+      const double jx = t[1][0][xl], jy = t[1][1][yl], jz = t[1][2][zl];
+      const double kx = t[2][0][xl], ky = t[2][1][yl], kz = t[2][2][zl];
+      u[0] -= ix * jk[gp[3]] + jy * ik[gp[1]] + kz * ij[gp[0]];
+      u[1] -= ix * jk[gp[5]] + jz * ik[gp[0]] + ky * ij[gp[1]];
+      u[2] -= iy * jk[gp[1]] + jx * ik[gp[3]] + kz * ij[gp[2]];
+      if (!PAIR) {
+        u[3] -= iy * jk[gp[4]] + jz * ik[gp[2]] + kx * ij[gp[3]];
+        u[4] -= iz * jk[gp[0]] + jx * ik[gp[5]] + ky * ij[gp[4]];
+        u[5] -= iz * jk[gp[2]] + jy * ik[gp[4]] + kx * ij[gp[5]];
+      }
+    }
+    // 1 / (d_i + d_j + d_k) of each permutation that an energy uses
+    const double dix = sd[0][0][xl], djx = sd[1][0][xl], dkx = sd[2][0][xl];
+    if (PAIR) {
+      // one triple: (f,s;f) of (ij;i), or (s,f;f) of (ij;j), whose W has the
+      // other sign and whose a lies at s; (y,z,x) = (x,z,y), (z,x,y) =
+      // (y,x,z), (z,y,x) = (x,y,z)
+      const bool sw = item.pad_ != 0;
+      const double d0 = sw ? (diy + djx) + dkz : (dix + djy) + dkz;
+      const double d1 = sw ? (diz + djx) + dky : (dix + djz) + dky;
+      const double d3 = sw ? (diz + djy) + dkx : (diy + djz) + dkx;
+      if (xy) e[0] += (u[0] - u[2]) * (w[0] - w[2]) * recip_nr(d0);
+      if (xy && yz) e[0] += (u[1] - u[2]) * (w[1] - w[2]) * recip_nr(d1);
+      if (yz) e[0] += (u[1] - u[0]) * (w[1] - w[0]) * recip_nr(d3);
+      continue;
+    }
+    const double r0 = recip_nr((dix + djy) + dkz);
+    const double r1 = recip_nr((dix + djz) + dky);
+    const double r2 = recip_nr((diy + djx) + dkz);
+    const double r3 = recip_nr((diy + djz) + dkx);
+    const double r4 = recip_nr((diz + djx) + dky);
     // (p - q) of U times (p - q) of W
     auto term = [&](int q, int n) { return (u[q] - u[n]) * (w[q] - w[n]); };
     if (xy && yz) {
@@ -227,31 +268,32 @@ __global__ void __launch_bounds__(GEPI_THREADS, 2)
   }
   // fixed-order sums over the CTA
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < (PAIR ? 1 : 4); ++q) {
 #pragma unroll
     for (int n = 16; n > 0; n >>= 1)
       e[q] += __shfl_down_sync(0xffffffffu, e[q], n);
     if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = e[q];
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (threadIdx.x < (PAIR ? 1 : 4)) {
     double s = 0.0;
     for (int n = 0; n < GEPI_THREADS / 32; ++n) s += red[threadIdx.x][n];
     item.partials[(int64_t)threadIdx.x * item.nblk + tile] = s;
   }
 }
 
-constexpr size_t GEPI_SMEM = (size_t)12 * PB * sizeof(double);
-
-template <bool FT, bool HASF>
+template <bool FT, bool HASF, bool PAIR>
 cudaError_t launch(const EpiItem *d_items, int grid, int nitems,
                    cudaStream_t st) {
+  constexpr size_t smem =
+      ((FT ? 2 : 1) * (PAIR ? 3 : 6) * PB + (HASF ? 36 : 18) * GB) *
+      sizeof(double);
   const cudaError_t e = cudaFuncSetAttribute(
-      epi_closed_kernel<FT, HASF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)GEPI_SMEM);
+      epi_closed_kernel<FT, HASF, PAIR>,
+      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  epi_closed_kernel<FT, HASF><<<dim3(grid, nitems), GEPI_THREADS, GEPI_SMEM,
-                                st>>>(d_items);
+  epi_closed_kernel<FT, HASF, PAIR>
+      <<<dim3(grid, nitems), GEPI_THREADS, smem, st>>>(d_items);
   return cudaGetLastError();
 }
 
@@ -343,14 +385,17 @@ __global__ void closed_check_oovo_kernel(const double *__restrict__ same,
 
 }  // namespace
 
-cudaError_t epi_closed_launch(const EpiItem *d_items, bool ft, bool hasf,
-                              int grid, int nitems, cudaStream_t st) {
+cudaError_t epi_closed_launch(const EpiItem *d_items, bool pair, bool ft,
+                              bool hasf, int grid, int nitems,
+                              cudaStream_t st) {
   if (grid <= 0 || nitems <= 0) return cudaSuccess;
-  if (ft)
-    return hasf ? launch<true, true>(d_items, grid, nitems, st)
-                : launch<true, false>(d_items, grid, nitems, st);
-  return hasf ? launch<false, true>(d_items, grid, nitems, st)
-              : launch<false, false>(d_items, grid, nitems, st);
+  using F = cudaError_t (*)(const EpiItem *, int, int, cudaStream_t);
+  constexpr F f[2][2][2] = {
+      {{launch<false, false, false>, launch<false, true, false>},
+       {launch<true, false, false>, launch<true, true, false>}},
+      {{launch<false, false, true>, launch<false, true, true>},
+       {launch<true, false, true>, launch<true, true, true>}}};
+  return f[pair][ft][hasf](d_items, grid, nitems, st);
 }
 
 cudaError_t closed_check_launch(const double *same, const double *mixed,

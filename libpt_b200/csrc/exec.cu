@@ -41,10 +41,11 @@ void Round::clear() {
       epi_blocks[a][f].clear();
       epi_hasf[a][f] = false;
     }
-  for (int f = 0; f < 2; ++f) {
-    grp[f].clear();
-    grp_hasf[f] = false;
-  }
+  for (int a = 0; a < 2; ++a)
+    for (int f = 0; f < 2; ++f) {
+      grp[a][f].clear();
+      grp_hasf[a][f] = false;
+    }
   red.clear();
   gemm_flops = 0.0;
   triples = 0;
@@ -121,7 +122,7 @@ void Executor::destroy() {
 size_t Executor::bytes_for(size_t triples, size_t jobs_per_triple,
                            bool graphs) {
   const size_t jobs = triples * jobs_per_triple * sizeof(GemmJob);
-  return HDR + 64 * (EXEC_MAX_GROUPS + 7) +
+  return HDR + 64 * (EXEC_MAX_GROUPS + 9) +
          (graphs ? EXEC_MAX_GROUPS : 1) * jobs +
          triples * (sizeof(EpiItem) + sizeof(RedItem));
 }
@@ -210,15 +211,15 @@ int Executor::launch_all(const std::vector<GemmGroup> &groups,
            : epi_aaa_launch(lst, items, f, hasf, grid, nitems, fixed, st_));
       if (launches) ++*launches;
     }
-  if (!fixed)
-    for (int f = 0; f < 2; ++f) {
-      if (r->grp[f].empty()) continue;
-      int grid = 0;
-      for (const EpiItem &it : r->grp[f]) grid = std::max(grid, it.nblk);
-      CK(epi_closed_launch(grp_items_[f], f, r->grp_hasf[f], grid,
-                           (int)r->grp[f].size(), st_));
-      if (launches) ++*launches;
-    }
+  for (int x = 0; !fixed && x < 4; ++x) {
+    const int a = x >> 1, f = x & 1;
+    if (r->grp[a][f].empty()) continue;
+    int grid = 0;
+    for (const EpiItem &it : r->grp[a][f]) grid = std::max(grid, it.nblk);
+    CK(epi_closed_launch(grp_items_[a][f], a, f, r->grp_hasf[a][f], grid,
+                         (int)r->grp[a][f].size(), st_));
+    if (launches) ++*launches;
+  }
   {
     const RedList *lst = reinterpret_cast<const RedList *>(d_buf_ + red_slot());
     int grid = fixed ? RED_GRID : std::min<int>(RED_GRID, (int)r->red.size());
@@ -285,12 +286,15 @@ int Executor::run(Round &r, unsigned *d_err, ExecTiming *timing,
       eoff[a][f] = off;
       off = align64(off + r.epi[a][f].size() * sizeof(EpiItem));
     }
-  size_t grp_off[2];
-  for (int f = 0; f < 2; ++f) {
-    grp_off[f] = off;
-    off = align64(off + r.grp[f].size() * sizeof(EpiItem));
-  }
-  if (graphs_ && (!r.grp[0].empty() || !r.grp[1].empty())) {
+  size_t grp_off[2][2];
+  bool grouped = false;
+  for (int a = 0; a < 2; ++a)
+    for (int f = 0; f < 2; ++f) {
+      grp_off[a][f] = off;
+      off = align64(off + r.grp[a][f].size() * sizeof(EpiItem));
+      grouped = grouped || !r.grp[a][f].empty();
+    }
+  if (graphs_ && grouped) {
     set_error("executor: closed-shell groups need direct launches");
     return LIBPT_ERR_ARG;
   }
@@ -334,11 +338,13 @@ int Executor::run(Round &r, unsigned *d_err, ExecTiming *timing,
                              : it.back().block_begin + r.epi_blocks[a][f].back();
       std::memcpy(h + epi_slot(a, f), &l, sizeof(l));
     }
-  for (int f = 0; f < 2; ++f) {
-    std::memcpy(h + grp_off[f], r.grp[f].data(),
-                r.grp[f].size() * sizeof(EpiItem));
-    grp_items_[f] = reinterpret_cast<const EpiItem *>(d_buf_ + grp_off[f]);
-  }
+  for (int a = 0; a < 2; ++a)
+    for (int f = 0; f < 2; ++f) {
+      std::memcpy(h + grp_off[a][f], r.grp[a][f].data(),
+                  r.grp[a][f].size() * sizeof(EpiItem));
+      grp_items_[a][f] =
+          reinterpret_cast<const EpiItem *>(d_buf_ + grp_off[a][f]);
+    }
   {
     std::memcpy(h + roff, r.red.data(), r.red.size() * sizeof(RedItem));
     RedList l;

@@ -47,8 +47,9 @@ struct Round {
   std::vector<EpiItem> epi[2][2];                   // [aab][ft], block_begin unset
   std::vector<int> epi_blocks[2][2];                // blocks of each item
   bool epi_hasf[2][2] = {};                         // some item's f_ov != 0
-  std::vector<EpiItem> grp[2];                      // closed-shell groups [ft]
-  bool grp_hasf[2] = {};                            // (direct launches only)
+  std::vector<EpiItem> grp[2][2];                   // closed-shell groups and
+  bool grp_hasf[2][2] = {};                         // pairs [pair][ft] (direct
+                                                    // launches only)
   std::vector<RedItem> red;
   double gemm_flops = 0.0;                          // reference flops
   size_t triples = 0;
@@ -106,7 +107,7 @@ class Executor {
   std::vector<const GemmJob *> gjobs_;   // device job arrays of the groups
   int epi_grid_[2][2] = {{0, 0}, {0, 0}};
   const EpiItem *epi_items_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-  const EpiItem *grp_items_[2] = {nullptr, nullptr};
+  const EpiItem *grp_items_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
 };
 
 }  // namespace ptb

@@ -19,6 +19,11 @@
 // (gemm_dmma.cu), and one epilogue adds the four energies (epi_closed.cu),
 // each into its triple's own slot.
 //
+// A mixed-spin triple with a repeated index, (ij;i) or (ij;j), needs three
+// products, 6 v^4 flops (8 v^4 by the general jobs): with f the repeated index
+// and s the other, A1 above for (f, s, f), which serves as A3 too, and
+//   Z[b][a][c] = Z_sff[b][a,c],  A2[b][a][c] = Z[b][a][c] + Z[b][c][a].
+//
 // The relations are measured on the device for every solve, on the operands
 // themselves: a solve (for the OVVV block: an occupied index) whose largest
 // deviation exceeds CLOSED_TOL times the block's largest element keeps the
@@ -81,7 +86,7 @@ bool holds(const unsigned long long *w) {
 // Whether a solve may run groups at all (its relations aside).
 bool closed_possible(const libpt_plan *p) {
   return !p->unrestricted && p->precision == LIBPT_PREC_FP64 &&
-         p->va >= CLOSED_MIN_V && p->oa >= 3;
+         p->va >= CLOSED_MIN_V && p->oa >= 2;
 }
 
 // The group case: views, job templates, epilogue tiles.
@@ -229,15 +234,15 @@ int closed_read(libpt_plan *p, cudaStream_t s, int upto) {
 }
 
 // Splits the entries of the whole queue whose largest occupied index lies in
-// [lo, hi) into groups (i < j < k, appended as packed triples) and the rest.
+// [lo, hi) into groups and pairs (queue entry, i, j, k; a pair's i == k or j ==
+// k) and the rest.
 void closed_split(const libpt_plan *p, int lo, int hi,
                   std::vector<int4> &groups, std::vector<int64_t> &rest) {
   const SpinCase *aaa = case_of(p, 0), *aab = case_of(p, 1);
   const int o = p->oa;
   auto grouped = [&](int i, int j, int k) {
-    return p->closed_on && i != j && j != k && i != k &&
-           p->closed_ok[(size_t)i] && p->closed_ok[(size_t)j] &&
-           p->closed_ok[(size_t)k];
+    return p->closed_on && p->closed_ok[(size_t)i] &&
+           p->closed_ok[(size_t)j] && p->closed_ok[(size_t)k];
   };
   int64_t q = aaa->first;
   for (int i = 0; i < o; ++i)
@@ -254,13 +259,16 @@ void closed_split(const libpt_plan *p, int lo, int hi,
     for (int j = i + 1; j < o; ++j)
       for (int k = 0; k < o; ++k, ++q) {
         const int top = std::max(j, k);
-        if (top < lo || top >= hi || grouped(i, j, k)) continue;
-        rest.push_back(q);
+        if (top < lo || top >= hi) continue;
+        if (!grouped(i, j, k))
+          rest.push_back(q);
+        else if (k == i || k == j)
+          groups.push_back(make_int4((int)q, i, j, k));
       }
 }
 
-// Appends groups to a round while they fit the plan's round resources;
-// *taken = groups appended.  A group counts as its four triples.
+// Appends groups and pairs to a round while they fit the plan's round
+// resources; *taken = those appended.  A group counts as its four triples.
 int closed_append(libpt_plan *p, const int4 *groups, size_t n, PlanCursor &cur,
                   Round &r, size_t *taken) {
   *taken = 0;
@@ -271,18 +279,28 @@ int closed_append(libpt_plan *p, const int4 *groups, size_t n, PlanCursor &cur,
   grp.kind = 3;
   grp.bm = c.bm;
   for (size_t t = 0; t < n; ++t) {
-    if (cur.triples + 4 > p->tri_cap || cur.ws + c.ws_stride > p->ws_cap ||
-        cur.part + 4 * (int64_t)c.ntiles > p->part_cap)
+    const int q = groups[t].x, k = groups[t].w;
+    const bool pair = k == groups[t].y || k == groups[t].z;
+    // a pair's occupied indices (f, s, f)
+    const bool swapped = k == groups[t].z;
+    const int ijk[3] = {pair && swapped ? groups[t].z : groups[t].y,
+                        pair && swapped ? groups[t].y : groups[t].z, k};
+    const int ne = pair ? 1 : 4;   // queue entries
+    if (cur.triples + ne > p->tri_cap || cur.ws + c.ws_stride > p->ws_cap ||
+        cur.part + ne * (int64_t)c.ntiles > p->part_cap)
       break;
-    const int q = groups[t].x, ijk[3] = {groups[t].y, groups[t].z, groups[t].w};
     double *ws = p->ws + cur.ws, *partials = p->partials + cur.part;
     cur.ws += c.ws_stride;
-    cur.part += 4 * (int64_t)c.ntiles;
-    cur.triples += 4;
+    cur.part += ne * (int64_t)c.ntiles;
+    cur.triples += ne;
     ++*taken;
     std::vector<GemmJob> &jobs = r.gemm[grp];
     const int map0 = r.maps[grp].add(c.d_maps, c.maps.m, MAX_MAPS);
-    for (const JobT &jt : c.jobs) {
+    for (size_t n = 0; n < c.jobs.size(); ++n) {
+      // a pair: rows f as they are, rows s without the transposed half, and
+      // the third array is the first
+      if (pair && n % 3 == 2) continue;
+      const JobT &jt = c.jobs[n];
       GemmJob g;
       std::memset(&g, 0, sizeof(g));
       g.out = ws + jt.off;
@@ -294,8 +312,8 @@ int closed_append(libpt_plan *p, const int4 *groups, size_t n, PlanCursor &cur,
       g.ntiles_n = ((jt.N + GRP_BY - 1) / GRP_BY) *
                    ((jt.N + GRP_BZ - 1) / GRP_BZ);
       g.mtiles = (jt.M + c.bm - 1) / c.bm;
-      g.nseg = jt.nseg;
-      for (int s = 0; s < jt.nseg; ++s) {
+      g.nseg = pair && n % 3 == 1 ? 2 : jt.nseg;
+      for (int s = 0; s < g.nseg; ++s) {
         const SegT &st = jt.seg[s];
         GemmSeg &gs = g.seg[s];
         gs.amap = st.amap;
@@ -318,21 +336,25 @@ int closed_append(libpt_plan *p, const int4 *groups, size_t n, PlanCursor &cur,
     e.j = ijk[1];
     e.k = ijk[2];
     e.nblk = c.ntiles;
-    r.grp[ft].push_back(e);
-    if (p->has_f) r.grp_hasf[ft] = true;
-    const int64_t slot[4] = {q, mixed_entry(p, first, ijk[0], ijk[1], ijk[2]),
-                             mixed_entry(p, first, ijk[0], ijk[2], ijk[1]),
-                             mixed_entry(p, first, ijk[1], ijk[2], ijk[0])};
-    for (int x = 0; x < 4; ++x) {
+    e.pad_ = swapped ? 1 : 0;
+    r.grp[pair][ft].push_back(e);
+    if (p->has_f) r.grp_hasf[pair][ft] = true;
+    for (int x = 0; x < ne; ++x) {
+      // a group's: its same-spin triple, then (ij;k), (ik;j), (jk;i)
+      const int64_t slot =
+          x == 0   ? q
+          : x == 1 ? mixed_entry(p, first, ijk[0], ijk[1], ijk[2])
+          : x == 2 ? mixed_entry(p, first, ijk[0], ijk[2], ijk[1])
+                   : mixed_entry(p, first, ijk[1], ijk[2], ijk[0]);
       RedItem red;
       red.partials = partials + (int64_t)x * c.ntiles;
-      red.dst = p->e_slot + slot[x];
+      red.dst = p->e_slot + slot;
       red.n = c.ntiles;
       red.pad_ = 0;
       r.red.push_back(red);
     }
-    r.gemm_flops += c.flops_per_triple;
-    r.triples += 4;
+    r.gemm_flops += pair ? case_of(p, 1)->flops_per_triple : c.flops_per_triple;
+    r.triples += ne;
   }
   return LIBPT_OK;
 }

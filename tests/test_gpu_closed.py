@@ -27,6 +27,7 @@ def plan_energy(case, dev):
 # v around the 8-wide index blocks, the 8 x 16 column tiles, the 16-row
 # fragments and 96- / 128-row tiles; o from the smallest group up
 @pytest.mark.parametrize("kind,o,v,fock", [
+    ("rpt", 2, 50, 0.0), ("rft", 2, 61, 1e-3),
     ("rpt", 3, 48, 0.0), ("rpt", 4, 49, 1e-3), ("rpt", 5, 50, 0.0),
     ("rpt", 3, 51, 1e-3), ("rpt", 4, 52, 0.0), ("rpt", 3, 55, 0.0),
     ("rpt", 9, 57, 1e-3), ("rpt", 4, 63, 0.0), ("rpt", 17, 64, 0.0),
