@@ -151,8 +151,8 @@ const char *libpt_last_error(void);
  * kernel (LIBPT_PREC_*, with the slice count in bits 8-14 for
  * LIBPT_PREC_EMU64, and bit 15 set for 8-bit digit planes -- a signed top
  * digit, unsigned lower digits; S <= 6 -- instead of 7-bit signed digits)
- * and bits 16-23 a tile variant: FP64 0 = 128-row,
- * 1 = 96-row tiles; emulated FP64 the index of one of the slice count's
+ * and bits 16-23 a tile variant: FP64 0 = 96-row,
+ * 1 = 48-row tiles; emulated FP64 the index of one of the slice count's
  * INT8 tile shapes (0 = widest); libpt_selftest_variants() counts them.
  * Bits 24-31 nonzero: the kernel reads its tensor maps from device memory
  * (the form batched multi-solve launches use) instead of kernel parameters.

@@ -15,12 +15,9 @@ namespace ptb {
 // OVVV/amplitude block (TMA view: dims (4, K, N/4, P)).  The slices are selected
 // by the occupied indices (Q, P) resp. (P) of the triple.
 
-constexpr int GEMM_BM = 128;   // rows of a CTA tile (96 or 128, per case)
 constexpr int GEMM_BN = 128;   // columns of a CTA tile
 constexpr int GEMM_BK = 16;    // contraction depth of one pipeline stage
 constexpr int GEMM_STAGES = 5;
-constexpr int GEMM_CONSUMER_WARPS = 8;
-constexpr int GEMM_THREADS = (GEMM_CONSUMER_WARPS + 1) * 32;
 constexpr int MAX_SEG = 6;
 constexpr int MAX_MAPS = 24;
 
@@ -94,7 +91,9 @@ struct GemmList {
 constexpr int GEMM_GRID = 148;
 
 size_t gemm_smem_bytes(int bm);
-// bm: CTA tile rows, 96 or 128 (the A views' box height must match).  The
+// Persistent grid of the DMMA kernels with tiles of bm rows.
+inline int dmma_grid(int bm) { return bm == 48 ? 2 * GEMM_GRID : GEMM_GRID; }
+// bm: CTA tile rows, 96 or 48 (the A views' box height must match).  The
 // kernels run `grid` persistent CTAs over the list's tiles.  Two forms:
 //   pm != null: the launch's tensor maps and the job / tile counts (njobs,
 //               ntiles) as kernel parameters (direct launches);

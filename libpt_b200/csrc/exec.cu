@@ -140,11 +140,13 @@ int Executor::launch_all(const std::vector<GemmGroup> &groups,
   int g = 0;
   for (const GemmGroup &grp : groups) {
     GemmList *lst = reinterpret_cast<GemmList *>(d_buf_ + gemm_slot(g));
-    int grid = GEMM_GRID;
+    const int most =
+        grp.kind == 0 || grp.kind == 3 ? dmma_grid(grp.bm) : GEMM_GRID;
+    int grid = most;
     if (!fixed) {
       int tiles = 0;
       for (const GemmJob &j : r->gemm.at(grp)) tiles += j.mtiles * j.ntiles_n;
-      grid = std::min(GEMM_GRID, tiles);
+      grid = std::min(most, tiles);
     }
     // direct launches whose views fit take them as kernel parameters
     const LaunchMaps *pm = nullptr;

@@ -6,13 +6,15 @@
 // its own sign) in one K loop, so the permuted contributions the reference
 // adds one GEMM at a time (e.g. src/pt.c:236-290) meet in the accumulator.
 //
-// Pipeline: warp 8 (one elected lane) stages A and B tiles with TMA into a
-// GEMM_STAGES-deep ring of shared-memory buffers guarded by mbarriers;
-// warps 0-7 run mma.sync.m16n8k4.f64 on (BM/2) x 32 warp tiles.
-// BM is 96 or 128 rows.  A job's last M tile multiplies only the 16-row
-// fragments that hold rows of the job, shared out to the two warp rows of the
-// tile: each has one warp on every SM sub-partition, so a tile's DMMA time
-// follows its fragment count (v = 143: 144 rows of work, not 192).
+// Pipeline: one elected lane of the last warp stages A and B tiles with TMA
+// into a GEMM_STAGES-deep ring of shared-memory buffers guarded by mbarriers;
+// the consumer warps run mma.sync.m16n8k4.f64 on 48 x 32 warp tiles.
+// BM is 96 rows (two warp rows, one CTA an SM) or 48 (one warp row, two CTAs
+// an SM, whose tile transitions hide behind each other); dmma_rows picks.  A
+// job's last M tile multiplies only the 16-row fragments that hold rows of the
+// job, shared out to the warp rows of the tile: each has one warp on every SM
+// sub-partition, so a tile's DMMA time follows its fragment count (v = 143: 144
+// rows of work, not 192).
 //
 // Shared-memory layouts (no swizzle; TMA box rows are 32 bytes):
 //   A stage [k/4][m][k%4]   -- one box of (4 k) x BM rows x 4
@@ -24,7 +26,7 @@
 // cycles, held a stage at 3.4 k cycles whatever its rows; 96 rows of DMMA
 // work take 3.1 k.
 //
-// Persistent: GEMM_GRID CTAs take the launch's tiles one at a time from the
+// Persistent: dmma_grid(BM) CTAs take the launch's tiles one at a time from the
 // tile queue of a device-memory work list (GemmList; common.cuh tq_*), so
 // one launch can hold the triples of many plans, tiles of uneven length
 // spread over the SMs, and a captured CUDA graph can be replayed with new
@@ -55,7 +57,15 @@ namespace ptb {
 namespace {
 
 constexpr int BN = GEMM_BN, BK = GEMM_BK, ST = GEMM_STAGES;
-constexpr int NCW = GEMM_CONSUMER_WARPS;
+
+// Consumer warps of a CTA: warp rows of 16 MF rows, four columns of 32.
+template <int BM>
+struct Dmma {
+  static constexpr int WR = BM > 64 ? 2 : 1;   // warp rows
+  static constexpr int MF = BM / (16 * WR);    // m16 fragments of a warp
+  static constexpr int NCW = 4 * WR;
+  static constexpr int THREADS = (NCW + 1) * 32;
+};
 
 template <int BM>
 constexpr uint32_t stage_bytes() {
@@ -101,16 +111,14 @@ __device__ __forceinline__ void mma_stage(double (&acc)[MF][4][4],
   }
 }
 
-// One CTA of GEMM_THREADS (9 warps) per SM.  With 9 warps one SM
-// sub-partition hosts 3 of them, which bounds the kernel at 168 registers per
-// thread (16K registers per sub-partition); the 128-row tile's 64 FP64
-// accumulators per thread fit that without spilling.
+// 9 or 10 warps an SM: one SM sub-partition hosts 3 of them, which bounds the
+// kernel at 168 registers per thread (16K registers per sub-partition).
 template <int BM, bool PM, bool GRP>
 __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
                                           const GemmJob *__restrict__ jobs,
                                           const int njobs, const int ntiles,
                                           GemmList *list, unsigned *err) {
-  constexpr int MF = BM / 32;   // m16 fragments per warp (2 warp rows)
+  constexpr int MF = Dmma<BM>::MF, NCW = Dmma<BM>::NCW, WR = Dmma<BM>::WR;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double *sA = reinterpret_cast<double *>(smem_raw);
   double *sB = sA + ST * BM * BK;
@@ -242,8 +250,8 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
         for (int e = 0; e < 4; ++e) acc[f][h][e] = 0.0;
     // the tile's 16-row fragments that hold rows of the job, shared out to
     // the two warp rows (a full tile: MF each)
-    const int frags = min(2 * MF, (job.M - m0 + 15) >> 4);
-    const int f0 = (frags + 1) >> 1;
+    const int frags = min(WR * MF, (job.M - m0 + 15) >> 4);
+    const int f0 = WR == 1 ? frags : (frags + 1) >> 1;
     const int nf = (warp >> 2) ? frags - f0 : f0;
     const int wm = (warp >> 2) ? 16 * f0 : 0;
     const int aoff = (wm + g) * 4 + t;
@@ -271,8 +279,6 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
           mma_stage<1, MF, BM>(acc, A, B, bo, mask, nkq);
         else if (nf == 2)
           mma_stage<2, MF, BM>(acc, A, B, bo, mask, nkq);
-        else if (MF == 4 && nf == 3)
-          mma_stage<3, MF, BM>(acc, A, B, bo, mask, nkq);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == ST) {
@@ -355,7 +361,7 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
 }
 
 template <int BM>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
     gemm_dmma_kernel(const __grid_constant__ LaunchMaps pm,
                      const GemmJob *__restrict__ jobs, int njobs, int ntiles,
                      GemmList *list, unsigned *err) {
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 }
 
 template <int BM>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
     gemm_dmma_kernel_dm(const GemmJob *__restrict__ jobs, GemmList *list,
                         unsigned *err) {
   dmma_body<BM, false, false>(nullptr, jobs, list->njobs, list->ntiles, list, err);
@@ -371,7 +377,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
 // Group jobs (direct launches only).
 template <int BM>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
     gemm_dmma_grp_kernel(const __grid_constant__ LaunchMaps pm,
                          const GemmJob *__restrict__ jobs, int njobs,
                          int ntiles, GemmList *list, unsigned *err) {
@@ -387,7 +393,7 @@ cudaError_t launch_grp(const GemmJob *d_jobs, GemmList *d_list, int njobs,
       gemm_dmma_grp_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
       (int)smem);
   if (e != cudaSuccess) return e;
-  gemm_dmma_grp_kernel<BM><<<grid, GEMM_THREADS, smem, st>>>(
+  gemm_dmma_grp_kernel<BM><<<grid, Dmma<BM>::THREADS, smem, st>>>(
       *pm, d_jobs, njobs, ntiles, d_list, d_err);
   return cudaGetLastError();
 }
@@ -410,11 +416,11 @@ cudaError_t launch(const GemmJob *d_jobs, GemmList *d_list, int njobs,
     configured = true;
   }
   if (pm)
-    gemm_dmma_kernel<BM><<<grid, GEMM_THREADS, smem, st>>>(*pm, d_jobs, njobs,
+    gemm_dmma_kernel<BM><<<grid, Dmma<BM>::THREADS, smem, st>>>(*pm, d_jobs, njobs,
                                                            ntiles, d_list,
                                                            d_err);
   else
-    gemm_dmma_kernel_dm<BM><<<grid, GEMM_THREADS, smem, st>>>(d_jobs, d_list,
+    gemm_dmma_kernel_dm<BM><<<grid, Dmma<BM>::THREADS, smem, st>>>(d_jobs, d_list,
                                                               d_err);
   return cudaGetLastError();
 }
@@ -431,9 +437,9 @@ cudaError_t gemm_dmma_launch(const GemmJob *d_jobs, GemmList *d_list,
                              int bm, int grid, unsigned *d_err,
                              cudaStream_t st) {
   if (grid <= 0) return cudaSuccess;
-  if (bm == 96)
-    return launch<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
-  return launch<128>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+  if (bm == 48)
+    return launch<48>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+  return launch<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
 }
 
 cudaError_t gemm_dmma_grp_launch(const GemmJob *d_jobs, GemmList *d_list,
@@ -442,9 +448,9 @@ cudaError_t gemm_dmma_grp_launch(const GemmJob *d_jobs, GemmList *d_list,
                                  cudaStream_t st) {
   if (grid <= 0) return cudaSuccess;
   if (!pm) return cudaErrorInvalidValue;
-  if (bm == 96)
-    return launch_grp<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
-  return launch_grp<128>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+  if (bm == 48)
+    return launch_grp<48>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
+  return launch_grp<96>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);
 }
 
 }  // namespace ptb

@@ -100,7 +100,7 @@ struct SpinCase {
   int ntiles = 0, ctiles = 0;
   CUtensorMap *d_maps = nullptr;        // the kernel's views, device memory
   double flops_per_triple = 0.0;        // reference GEMM flops
-  int bm = GEMM_BM;                     // CTA tile rows of this case's GEMMs
+  int bm = 96;                          // CTA tile rows of this case's GEMMs
   OpDesc opd[MAX_MAPS];                 // operand behind each DMMA map
   TcMapSet tcmaps;                      // tensor-core views (TF32: map 2i,
                                         // 2i+1; emulated FP64: map i)

@@ -328,20 +328,15 @@ int build_aab(libpt_plan *p, SpinCase &c) {
   return LIBPT_OK;
 }
 
-// Modelled SM cycles per 16-deep K step of the tile column that covers m
-// rows with tiles of bm rows: the kernel multiplies whole 16-row fragments
-// (64 FP64 multiply-adds per cycle: 32 cycles per row of a 128-column tile),
-// and a tile cannot run faster than its operands arrive (26 bytes per cycle
-// with 32-byte TMA box rows).  Only a last tile of 16 rows is bound by its
-// operands, so 97..112 rows go to one 128-row tile, not to 96 + 16.
-int64_t dmma_row_cost(int64_t m, int64_t bm) {
-  int64_t cost = 0;
-  for (int64_t r = 0; r < m; r += bm) {
-    const int64_t rows = (std::min(bm, m - r) + 15) / 16 * 16;
-    cost += std::max<int64_t>(32 * rows, (rows + GEMM_BN) * GEMM_BK * 8 / 26);
-  }
-  return cost;
-}
+// DMMA tile rows for jobs of m rows: 96, or 48 with two CTAs an SM.  Both
+// multiply the same 16-row fragments.  A 48-row tile moves 1.6 times the
+// operand bytes per product, but one CTA's stores run beside the other's
+// products, where a 96-row CTA's are exposed; what decides is the last tile,
+// of which a 96-row CTA with at most 48 rows makes two fragments or fewer a
+// warp.  Mixed-spin probes, 48 against 96 rows: v = 104 0.93, 143 0.94, 201
+// and 240 0.96, 300 0.97 of the time; v = 64 to 90 1.03 and more, 160 and 180
+// 1.01, 477 1.01.
+int dmma_rows(int64_t m) { return m > 96 && (m - 1) % 96 < 48 ? 48 : 96; }
 
 int add_cases(libpt_plan *p) {
   const int oa = p->oa, va = p->va, ob = p->ob, vb = p->vb;
@@ -380,13 +375,7 @@ int add_cases(libpt_plan *p) {
   if (p->unrestricted) add(1, 1, ob, vb, oa, va);
   for (SpinCase &c : p->cases) {
     if (c.count == 0) continue;
-    // CTA tile rows: the least modelled time of the GEMM rows (va, and vb
-    // for the mixed-spin P job); ties go to 96 (no register spills)
-    const int64_t w128 = dmma_row_cost(c.va, 128) +
-                         (c.type ? dmma_row_cost(c.vb, 128) : 0);
-    const int64_t w96 = dmma_row_cost(c.va, 96) +
-                        (c.type ? dmma_row_cost(c.vb, 96) : 0);
-    c.bm = w128 < w96 ? 128 : 96;
+    c.bm = dmma_rows(c.va);
     int r = c.type == 0 ? build_aaa(p, c) : build_aab(p, c);
     if (!r && p->precision == LIBPT_PREC_TF32X3) r = build_tc(p, c);
     if (r) return r;

@@ -97,7 +97,7 @@ int closed_build(libpt_plan *p) {
   c.type = 2;
   c.oa = c.ob = (int)o;
   c.va = c.vb = (int)v;
-  c.bm = dmma_row_cost(v, 128) < dmma_row_cost(v, 96) ? 128 : 96;
+  c.bm = dmma_rows(v);
   EpiArgs &e = c.epi;
   std::memset(&e, 0, sizeof(e));
   int64_t stride = 0;

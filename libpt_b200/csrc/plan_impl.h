@@ -188,8 +188,8 @@ int flush_deferred(libpt_plan *p);
 // ---- spin cases, job templates, queue (plan_cases.cu) -----------------------
 int add_cases(libpt_plan *p);
 SegT seg(int amap, int bmap, bool neg, int aq, int ap, int bp, int64_t k);
-// Modelled cost of m rows in DMMA tiles of bm rows.
-int64_t dmma_row_cost(int64_t m, int64_t bm);
+// DMMA tile rows (96 or 48) for jobs of m rows.
+int dmma_rows(int64_t m);
 // Copies each case's kernel views (tensor maps) and epilogue arguments to
 // device memory, where the kernels read them.  Re-run after any map change.
 int upload_views(libpt_plan *p);

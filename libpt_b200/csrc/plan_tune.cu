@@ -47,7 +47,7 @@ int set_bm(SpinCase &c, int bm) {
 // The autotuner: picks the kernel variants of a plan by timing them on a
 // probe of its triples (each candidate run twice, the second run timed),
 // and remembers the choice per (kind, sizes, precision, slices, dtype).
-//   FP64 DMMA:      CTA tile rows 96 or 128, per spin case
+//   FP64 DMMA:      CTA tile rows 96 or 48, per spin case
 //   emulated FP64:  the INT8 tile variants of the slice count (i8_tiles)
 // The probe's energies are discarded (slots reset afterwards); choices do
 // not change results, only speed (each output element is accumulated in
@@ -98,7 +98,7 @@ int autotune(libpt_plan *p) {
           if (int r = i8_encode(p, c)) return r;
     } else if (!emu && choice.size() == p->cases.size()) {
       for (size_t ci = 0; ci < p->cases.size(); ++ci)
-        if (p->cases[ci].count && (choice[ci] == 96 || choice[ci] == 128))
+        if (p->cases[ci].count && (choice[ci] == 48 || choice[ci] == 96))
           if (int r = set_bm(p->cases[ci], choice[ci])) return r;
     }
     return upload_views(p);
@@ -169,7 +169,7 @@ int autotune(libpt_plan *p) {
       const int start = c.bm;
       int best = start;
       float best_ms = 0.f;
-      for (int bm : {start, start == 96 ? 128 : 96}) {
+      for (int bm : {start, start == 48 ? 96 : 48}) {
         if ((r = set_bm(c, bm))) break;
         if ((r = upload_views(p))) break;
         float ms = 0.f;

@@ -157,7 +157,9 @@ int kernel_case(int precision, int m, int n, int k, int reps, double *rel_err,
     l.njobs = 1;
     l.ntiles = job.mtiles * job.ntiles_n;
     nt = l.ntiles;
-    grid = l.ntiles < GEMM_GRID ? l.ntiles : GEMM_GRID;
+    const int most =
+        precision == LIBPT_PREC_FP64 ? dmma_grid(variant ? 48 : 96) : GEMM_GRID;
+    grid = l.ntiles < most ? l.ntiles : most;
     cudaMemcpy(dmaps, maps, bytes, cudaMemcpyHostToDevice);
     cudaMemcpy(dj, &job, sizeof(job), cudaMemcpyHostToDevice);
     cudaMemcpy(dl, &l, sizeof(l), cudaMemcpyHostToDevice);
@@ -165,7 +167,7 @@ int kernel_case(int precision, int m, int n, int k, int reps, double *rel_err,
   if (precision == LIBPT_PREC_FP64) {
     MapSet maps;
     memset(&maps, 0, sizeof(maps));
-    const int bm = variant ? 96 : 128;
+    const int bm = variant ? 48 : 96;
     if ((r = dmma_map_a(&maps.m[0], A, k, m, 1, 1, bm)) ||
         (r = dmma_map_b(&maps.m[1], B1, n, np, k, 1)) ||
         (r = dmma_map_b(&maps.m[2], B2, n, np, k, 1)))
