@@ -349,7 +349,7 @@ size_t plan_footprint(int kind, size_t oa, size_t va, size_t ob, size_t vb,
 
 void plan_destroy(libpt_plan *p) {
   if (!p) return;
-  if (p->st) cudaStreamSynchronize(p->st);
+  if (p->st || !p->allocs.empty()) cudaStreamSynchronize(p->st);
   if (p->st_up) {
     cudaStreamSynchronize(p->st_up);
     cudaStreamDestroy(p->st_up);
@@ -361,7 +361,7 @@ void plan_destroy(libpt_plan *p) {
   if (p->exec_ready) p->exec.destroy();
   // the caller may read the energy slots on streams of its own
   if (p->slots_shared) cudaDeviceSynchronize();
-  while (!p->allocs.empty()) dfree(p, p->allocs.back());
+  while (!p->allocs.empty()) dfree(p, p->allocs.back().p);
   delete p;
 }
 

@@ -73,6 +73,13 @@ struct JobT {
   const signed char *ea = nullptr, *eb = nullptr;   // emulated FP64 scales
 };
 
+// A device buffer of a plan, and the context it was made in.
+struct DeviceBuffer {
+  void *p;
+  size_t n;
+  uint64_t ctx;
+};
+
 // Padded device copies of one amplitude + integral set (index 0 aaaa,
 // 1 abab, 2 bbbb, 3 baba; packed pairs 0 aaaa, 1 bbbb).
 struct OperandSet {
@@ -134,8 +141,7 @@ struct libpt_plan {
   cudaStream_t st_rd = nullptr;   // reads the rows' closed-shell checks
   void *up_stage[2] = {nullptr, nullptr};
   size_t up_stage_bytes = 0;
-  std::vector<void *> allocs;           // device buffers (no arena)
-  std::vector<void *> pooled;           // ... those of the library's pool
+  std::vector<ptb::DeviceBuffer> allocs;   // device buffers (no arena)
   ptb::OperandSet L, R;
   double *d_ov = nullptr, *ov1 = nullptr, *ov2 = nullptr;
   bool has_f = true;                    // f_ov / f2_ov not all zero

@@ -44,10 +44,10 @@ int map_f64(CUtensorMap *m, const double *p, int rank, const int64_t *dims,
 int build_tc(libpt_plan *p, SpinCase &c);
 
 // ---- device memory and uploads (plan_upload.cu) -----------------------------
-// A device buffer of the plan: carved from its arena, or allocated from the
-// library's memory pool and freed with the plan.
+// A device buffer of the plan: carved from its arena, or taken from the
+// buffers kept between solves or cudaMalloc, and given back with the plan.
 int dalloc(libpt_plan *p, void **ptr, size_t bytes);
-// Frees one of them early (nothing for an arena's), ordered on the plan's
+// Gives one of them back early (nothing for an arena's), after the plan's
 // stream.
 void dfree(libpt_plan *p, void *ptr);
 

@@ -42,13 +42,16 @@ int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
   // per GB, each round some 50 us of launches and a partial last wave, so the
   // sum is least near 0.19 sqrt(outputs in GB) GB; at least 1 GiB (a round of
   // that size is long enough), at most the budget.  (o = 14, v = 143, 47 GB
-  // of outputs: 24 ms of the solve went to a 16 GiB workspace.)
-  double want_all = std::min(
-      total, std::max((double)((size_t)1 << 30), 0.19e9 * std::sqrt(total * 8e-9)) / 8);
+  // of outputs: 24 ms of the solve went to a 16 GiB workspace.)  Up to 2 GiB
+  // a workspace of 1 GiB, which is kept between solves, is the better choice.
+  const double gib = (double)((size_t)1 << 30);
+  double best = 0.19e9 * std::sqrt(total * 8e-9);
+  if (best < 2.0 * gib) best = gib;
+  double want_all = std::min(total, best / 8);
   // beyond 2 GiB: no more than half of what is free, nor than 16 GiB (the
   // query itself can take milliseconds; smaller workspaces are halved below
   // where they do not fit)
-  if (!p->arena && want_all * 8 > (double)((size_t)2 << 30)) {
+  if (!p->arena && want_all * 8 >= 2.0 * gib) {
     if (!p->ws_budget) {
       size_t fr = 0, tot = 0;
       cudaMemGetInfo(&fr, &tot);

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <list>
 #include <string>
 #include <vector>
 
@@ -21,45 +22,113 @@ namespace ptb {
 
 namespace {
 
-// The library's memory pool of the current device (null where the device has
-// none).  A solve has 20 to 80 device buffers, and a cudaMalloc / cudaFree
-// pair takes 0.7 ms and more (2 MB: 0.4 + 0.3, 1 GB: 0.7 + 1.0): 8 of 10 ms of
-// a host-array solve at o = 8, v = 64.  The pool holds at most POOL_BYTES
-// (1.1 % of the device's memory) and keeps them between solves; it gives them
-// back when an allocation of the library fails.  What does not fit comes from
-// cudaMalloc: growing and trimming a pool costs 5 ms per GB each way, five to
-// ten times as much.  Its allocations and frees are ordered by the streams
-// that make them, so any threads and streams may share it.
-constexpr size_t POOL_BYTES = (size_t)2 << 30;
+// Device buffers kept between solves.  A solve has 20 to 80 of them, and a
+// cudaMalloc / cudaFree pair takes 0.7 ms and more (2 MB: 0.4 + 0.3, 1 GB: 0.7 +
+// 1.0): 8 of 10 ms of a host-array solve at o = 8, v = 64.  At most KEEP_BYTES
+// (1.1 % of the device's memory) are kept, the rest given up, and all of them
+// when an allocation of the library fails.  A buffer comes back only after the
+// stream that used it has been waited for, so any thread and stream may take it
+// next.  Buffers belong to the context they were made in (its process-wide id:
+// a reset device has a new one, and nothing of the old is handed out).  A CUDA
+// memory pool was measured instead: it maps and unmaps at 5 ms per GB each way
+// whenever the buffers of two solves do not fit its free space alike (FP32 upt
+// 12/120/11/122: 58 to 200 ms a call).
+constexpr size_t KEEP_BYTES = (size_t)2 << 30;
+constexpr size_t KEEP_BUFFER = (size_t)1280 << 20;   // larger ones are not kept
 
-cudaMemPool_t device_pool() {
-  static std::mutex mu;
-  static std::vector<std::pair<int, cudaMemPool_t>> pools;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  std::lock_guard<std::mutex> g(mu);
-  for (auto &e : pools)
-    if (e.first == dev) return e.second;
-  cudaMemPool_t pool = nullptr;
-  int has = 0;
-  if (cudaDeviceGetAttribute(&has, cudaDevAttrMemoryPoolsSupported, dev) ==
-          cudaSuccess &&
-      has) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    props.maxSize = POOL_BYTES;
-    uint64_t keep = POOL_BYTES;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
-      pool = nullptr;
-    else
-      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+class BufferCache {
+ public:
+  static BufferCache &get() {
+    static BufferCache *c = new BufferCache();   // outlives every plan
+    return *c;
   }
-  cudaGetLastError();
-  pools.push_back({dev, pool});
-  return pool;
-}
+
+  // 0: unknown (nothing is kept)
+  static uint64_t context() {
+    typedef CUresult (*GetId)(CUcontext, unsigned long long *);
+    static GetId fn = [] {
+      void *p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      return cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) ==
+                         cudaSuccess &&
+                     q == cudaDriverEntryPointSuccess
+                 ? reinterpret_cast<GetId>(p)
+                 : nullptr;
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+  }
+
+  // whole 64 KiB (2 MiB from there on), so that sizes of like solves meet
+  static size_t rounded(size_t n) {
+    const size_t g = n <= ((size_t)2 << 20) ? (size_t)64 << 10 : (size_t)2 << 20;
+    return (n + g - 1) & ~(g - 1);
+  }
+
+  // The smallest kept buffer of n bytes or little more, or null.
+  void *take(uint64_t ctx, size_t n, size_t *size) {
+    std::lock_guard<std::mutex> g(mu_);
+    auto best = kept_.end();
+    for (auto it = kept_.begin(); it != kept_.end(); ++it)
+      if (it->ctx == ctx && it->n >= n && it->n <= n + n / 4 + ((size_t)1 << 20) &&
+          (best == kept_.end() || it->n < best->n))
+        best = it;
+    if (best == kept_.end()) return nullptr;
+    void *p = best->p;
+    *size = best->n;
+    bytes_ -= best->n;
+    kept_.erase(best);
+    return p;
+  }
+
+  // Keeps a buffer nothing on the device uses any more (of the current
+  // context ctx), giving up the oldest ones beyond KEEP_BYTES.
+  void give(uint64_t ctx, void *p, size_t n) {
+    std::vector<void *> drop;
+    if (n > KEEP_BUFFER) {
+      drop.push_back(p);
+    } else {
+      std::lock_guard<std::mutex> g(mu_);
+      kept_.push_front({ctx, p, n, ++gives_});
+      bytes_ += n;
+      while (bytes_ > KEEP_BYTES) {
+        // the oldest if it has lain unused for long, else the largest: a
+        // solve that outgrows the cache then allocates few buffers anew
+        auto out = std::prev(kept_.end());
+        if (gives_ - out->at < 512)
+          for (auto it = kept_.begin(); it != kept_.end(); ++it)
+            if (it->n > out->n) out = it;
+        if (out->ctx == ctx) drop.push_back(out->p);   // else gone with it
+        bytes_ -= out->n;
+        kept_.erase(out);
+      }
+    }
+    for (void *q : drop) cudaFree(q);
+  }
+
+  void give_up_all(uint64_t ctx) {
+    std::list<Kept> all;
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      all.swap(kept_);
+      bytes_ = 0;
+    }
+    for (const Kept &k : all)
+      if (k.ctx == ctx) cudaFree(k.p);
+  }
+
+ private:
+  struct Kept {
+    uint64_t ctx;
+    void *p;
+    size_t n;
+    uint64_t at;   // gives_ when it was given
+  };
+  std::mutex mu_;
+  std::list<Kept> kept_;   // most recently given first
+  size_t bytes_ = 0;
+  uint64_t gives_ = 0;
+};
 
 }  // namespace
 
@@ -77,44 +146,44 @@ int dalloc(libpt_plan *p, void **ptr, size_t bytes) {
     p->arena_used = off + bytes;
     return LIBPT_OK;
   }
-  const cudaMemPool_t pool = device_pool();
-  if (pool && bytes <= POOL_BYTES) {
-    if (cudaMallocFromPoolAsync(ptr, bytes, pool, p->st) == cudaSuccess) {
-      p->allocs.push_back(*ptr);
-      p->pooled.push_back(*ptr);
-      return LIBPT_OK;
+  BufferCache &cache = BufferCache::get();
+  const uint64_t ctx = BufferCache::context();
+  size_t n = BufferCache::rounded(bytes);
+  if (ctx) *ptr = cache.take(ctx, n, &n);
+  if (!*ptr) {
+    cudaError_t e = cudaMalloc(ptr, n);
+    if (e == cudaErrorMemoryAllocation && ctx) {
+      cudaGetLastError();
+      cache.give_up_all(ctx);
+      n = bytes;
+      e = cudaMalloc(ptr, n);
     }
-    cudaGetLastError();   // the pool is full
+    if (e != cudaSuccess) {
+      *ptr = nullptr;
+      set_error("cudaMalloc(" + std::to_string(bytes) +
+                " bytes): " + cudaGetErrorString(e));
+      cudaGetLastError();
+      return LIBPT_ERR_NOMEM;
+    }
   }
-  cudaError_t e = cudaMalloc(ptr, bytes);
-  if (e == cudaErrorMemoryAllocation && pool) {
-    // what the pool keeps from earlier solves goes back first
-    cudaGetLastError();
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
-    e = cudaMalloc(ptr, bytes);
-  }
-  if (e != cudaSuccess) {
-    set_error("device allocation (" + std::to_string(bytes) +
-              " bytes): " + cudaGetErrorString(e));
-    cudaGetLastError();
-    return LIBPT_ERR_NOMEM;
-  }
-  p->allocs.push_back(*ptr);
+  p->allocs.push_back({*ptr, n, ctx});
   return LIBPT_OK;
 }
 
 void dfree(libpt_plan *p, void *ptr) {
-  auto it = std::find(p->allocs.begin(), p->allocs.end(), ptr);
-  if (it == p->allocs.end()) return;   // carved from an arena
-  p->allocs.erase(it);
-  auto po = std::find(p->pooled.begin(), p->pooled.end(), ptr);
-  if (po != p->pooled.end()) {
-    p->pooled.erase(po);
-    if (cudaFreeAsync(ptr, p->st) == cudaSuccess) return;
-    cudaGetLastError();   // another device is current by now
+  for (auto it = p->allocs.begin(); it != p->allocs.end(); ++it) {
+    if (it->p != ptr) continue;   // (not found: carved from an arena)
+    const DeviceBuffer b = *it;
+    p->allocs.erase(it);
+    // nothing still runs on it (or the context is broken, or another one is
+    // current: then it is not kept)
+    if (b.ctx && cudaStreamSynchronize(p->st) == cudaSuccess &&
+        b.ctx == BufferCache::context())
+      BufferCache::get().give(b.ctx, b.p, b.n);
+    else
+      cudaFree(b.p);
+    return;
   }
-  cudaFree(ptr);
 }
 
 PinnedRing &pinned_ring() {
