@@ -175,7 +175,11 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
     p->up_stage[1] = up.stage[1];
     p->up_stage_bytes = up.stage_bytes;
     p->closed_want = solve && closed_possible(p);
-    if (p->closed_want && (r = closed_check(p))) break;
+    if (p->closed_want && (r = closed_check(p))) {
+      if (r != LIBPT_ERR_NOMEM) break;
+      r = LIBPT_OK;   // no room for the check's words: general jobs
+      p->closed_want = false;
+    }
     if (!g_dry && cudaStreamSynchronize(st) != cudaSuccess) {
       set_error(std::string("preparing operands: ") +
                 cudaGetErrorString(cudaGetLastError()));
@@ -201,7 +205,11 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
         break;
     }
     if ((r = add_cases(p))) break;
-    if (p->closed_want && p->closed_on && (r = closed_build(p))) break;
+    if (p->closed_want && p->closed_on && (r = closed_build(p))) {
+      if (r != LIBPT_ERR_NOMEM) break;
+      r = LIBPT_OK;
+      p->closed_on = false;
+    }
     if (p->precision != LIBPT_PREC_FP64) {
       // the tensor-core paths read planes; of the padded FP64 blocks only the
       // amplitudes stay (the energy epilogue's disconnected term reads them)
