@@ -300,11 +300,15 @@ int libpt_rpt_dev_static(size_t oa, size_t va, const double *d_ov,
  * (unrestricted only) -- the order of src/pt.c:514-529.  Running every queue
  * entry once and calling libpt_plan_energy gives the solver's result
  * (including the restricted factor 2, src/pt.c:478): the same bits, but for
- * restricted FP64 solves of v >= 48 whose same-spin blocks are the
- * antisymmetrised mixed-spin ones to rounding.  The one-call entry points
- * form the products those inputs share between the triples of {i, j, k}
- * once; a plan, whose entries may run in any pieces, does not, and the two
- * agree to rounding.
+ * restricted FP64 solves of v >= 48 whose same-spin blocks are exactly the
+ * antisymmetrised mixed-spin ones (every element the FP64 difference of its
+ * two).  The one-call entry points form the products those inputs share
+ * between the triples of {i, j, k} once; a plan, whose entries may run in any
+ * pieces, does not, and the two agree to rounding.  With LIBPT_CLOSED_TOL=x
+ * in the environment the one-call solves do the same for blocks that differ
+ * by up to x times the block's largest element (integrals transformed block
+ * by block: about 1e-13); the same-spin blocks are then not read, and the
+ * energy changes by a relative amount of that order.
  *
  * kind: 0 = (T) restricted, 1 = (T) unrestricted, 2 = (fT) restricted,
  *       3 = (fT) unrestricted.

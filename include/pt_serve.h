@@ -23,8 +23,8 @@
  *    (per-triple energies in fixed order, summed in queue order): bitwise,
  *    whatever else shares its rounds.  libpt_{r,u}{pt,ft} return the same
  *    bits except for restricted FP64 inputs of v >= 48 whose same-spin
- *    blocks are the antisymmetrised mixed-spin ones: those solves add the
- *    same products in another order and agree to rounding.
+ *    blocks are exactly the antisymmetrised mixed-spin ones: those solves add
+ *    the same products in another order and agree to rounding.
  */
 #ifndef LIBPT_PT_SERVE_H
 #define LIBPT_PT_SERVE_H

@@ -174,6 +174,7 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
     p->up_stage[0] = up.stage[0];   // for the deferred OVVV copies
     p->up_stage[1] = up.stage[1];
     p->up_stage_bytes = up.stage_bytes;
+    p->closed_tol = closed_tol();
     p->closed_want = solve && closed_possible(p);
     if (p->closed_want && (r = closed_check(p))) {
       if (r != LIBPT_ERR_NOMEM) break;

@@ -190,6 +190,7 @@ struct libpt_plan {
   ptb::ExecTiming tm;
   int64_t launches = 0;                      // kernels launched by runs
   // closed-shell groups of a restricted one-call solve (plan_closed.cu)
+  double closed_tol = 0.0;                   // allowed deviation (0: none)
   bool closed_want = false;                  // created for plan_run_solve
   bool closed_on = false;                    // the relations hold
   std::vector<char> closed_ok;               // ... of each occupied index

@@ -25,20 +25,25 @@
 //   Z[b][a][c] = Z_sff[b][a,c],  A2[b][a][c] = Z[b][a][c] + Z[b][c][a].
 //
 // The relations are measured on the device for every solve, on the operands
-// themselves: a solve (for the OVVV block: an occupied index) whose largest
-// deviation exceeds CLOSED_TOL times the block's largest element keeps the
-// general jobs.  Integrals transformed in FP64 satisfy them to a few
-// rounding errors of the largest element (5e-14 of it in the reference's
-// own fixtures); 2^-43 leaves the energy's change by the choice of block far
-// below its own rounding bound.
+// themselves, and have to hold exactly: every same-spin element the FP64
+// difference of its two mixed-spin ones, t_ij[ab] the same number as t_ji[ba]
+// (for the OVVV block: by occupied index).  Then the groups read what the
+// caller passed, up to that difference's own rounding, and the energy's error
+// stays the general jobs' (1e-16 of the same-spin energy, o = 3, v = 48,
+// against 80-bit sums).  A bound on the deviation does not keep it: blocks
+// that differ by 2^-43 of the largest element, which integrals transformed
+// block by block in FP64 do (5e-14 of it in the reference's own fixtures),
+// move that energy by 8.5e-15 (random deviations) to 2.7e-13 (a common
+// factor), because the groups read the mixed-spin blocks in place of the
+// same-spin ones.  A caller who accepts that names the bound in
+// LIBPT_CLOSED_TOL (closed_tol).
 //
 // Only the one-call solves run groups: plans and shards run any subset of
 // the queue and promise the same bits for every split, so a triple's
-// arithmetic there must not depend on which others run beside it.  Small
-// spaces (v < CLOSED_MIN_V) keep the general jobs: 8 x 16 column tiles pad
-// them more than the flops saved.
+// arithmetic there must not depend on which others run beside it.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -47,8 +52,6 @@
 namespace ptb {
 
 namespace {
-
-constexpr double CLOSED_TOL = 0x1p-43;
 
 // Views of an operand block [P][K][v][v4] as a group job's B: dims
 // (4, K, first index, quads of the second, P) with a box of one stage.
@@ -74,14 +77,21 @@ const SpinCase *case_of(const libpt_plan *p, int type) {
   return nullptr;
 }
 
-bool holds(const unsigned long long *w) {
+bool holds(const libpt_plan *p, const unsigned long long *w) {
   double dev, mag;
   std::memcpy(&dev, &w[0], 8);
   std::memcpy(&mag, &w[1], 8);
-  return std::isfinite(dev) && std::isfinite(mag) && dev <= CLOSED_TOL * mag;
+  return std::isfinite(dev) && std::isfinite(mag) && dev <= p->closed_tol * mag;
 }
 
 }  // namespace
+
+// Largest deviation from the relations, as a share of the block's largest
+// element, that a solve may run groups with.
+double closed_tol() {
+  const char *t = std::getenv("LIBPT_CLOSED_TOL");
+  return t ? std::max(std::atof(t), 0.0) : 0.0;
+}
 
 // Whether a solve may run groups at all (its relations aside).
 bool closed_possible(const libpt_plan *p) {
@@ -220,14 +230,15 @@ int closed_read(libpt_plan *p, cudaStream_t s, int upto) {
                      cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   const unsigned long long *w = words.data();
-  p->closed_on = holds(w);
+  p->closed_on = holds(p, w);
   for (int x = 0; x < nset; ++x)
-    p->closed_on = p->closed_on && holds(w + 2 + 4 * x) && holds(w + 4 + 4 * x);
+    p->closed_on = p->closed_on && holds(p, w + 2 + 4 * x) &&
+                   holds(p, w + 4 + 4 * x);
   p->closed_ok.assign((size_t)p->oa, 0);
   for (int i = 0; i < upto; ++i) {
     bool ok = true;
     for (int x = 0; x < nset; ++x)
-      ok = ok && holds(w + 16 + 2 * (x * p->oa + i));
+      ok = ok && holds(p, w + 16 + 2 * (x * p->oa + i));
     p->closed_ok[(size_t)i] = ok;
   }
   return LIBPT_OK;

@@ -217,6 +217,7 @@ int run_entries(libpt_plan *p, const std::vector<int64_t> &ents);
 // ---- closed-shell triples (plan_closed.cu) ----------------------------------
 // Smallest v whose restricted solves run groups.
 constexpr int CLOSED_MIN_V = 48;
+double closed_tol();
 bool closed_possible(const libpt_plan *p);
 int closed_build(libpt_plan *p);
 int closed_check(libpt_plan *p);
