@@ -308,7 +308,9 @@ int libpt_rpt_dev_static(size_t oa, size_t va, const double *d_ov,
  * in the environment the one-call solves do the same for blocks that differ
  * by up to x times the block's largest element (integrals transformed block
  * by block: about 1e-13); the same-spin blocks are then not read, and the
- * energy changes by a relative amount of that order.
+ * energy changes by a relative amount of that order.  With a negative x they
+ * never do, and every energy of one solve -- one-call, plan, shards, served --
+ * has the same bits.
  *
  * kind: 0 = (T) restricted, 1 = (T) unrestricted, 2 = (fT) restricted,
  *       3 = (fT) unrestricted.

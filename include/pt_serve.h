@@ -24,7 +24,8 @@
  *    whatever else shares its rounds.  libpt_{r,u}{pt,ft} return the same
  *    bits except for restricted FP64 inputs of v >= 48 whose same-spin
  *    blocks are exactly the antisymmetrised mixed-spin ones: those solves add
- *    the same products in another order and agree to rounding.
+ *    the same products in another order and agree to rounding, or to the
+ *    bit with LIBPT_CLOSED_TOL=-1 in the environment (pt.h).
  */
 #ifndef LIBPT_PT_SERVE_H
 #define LIBPT_PT_SERVE_H

@@ -87,15 +87,17 @@ bool holds(const libpt_plan *p, const unsigned long long *w) {
 }  // namespace
 
 // Largest deviation from the relations, as a share of the block's largest
-// element, that a solve may run groups with.
+// element, that a solve may run groups with; negative: none does, and its
+// energy is a plan's bit for bit.
 double closed_tol() {
   const char *t = std::getenv("LIBPT_CLOSED_TOL");
-  return t ? std::max(std::atof(t), 0.0) : 0.0;
+  return t ? std::atof(t) : 0.0;
 }
 
 // Whether a solve may run groups at all (its relations aside).
 bool closed_possible(const libpt_plan *p) {
-  return !p->unrestricted && p->precision == LIBPT_PREC_FP64 &&
+  return p->closed_tol >= 0.0 && !p->unrestricted &&
+         p->precision == LIBPT_PREC_FP64 &&
          p->va >= CLOSED_MIN_V && p->oa >= 2;
 }
 
