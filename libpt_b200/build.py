@@ -32,7 +32,7 @@ SOURCES = ["gemm_dmma.cu", "gemm_tc.cu", "gemm_i8.cu", "epilogue.cu", "epi_close
            "tune.cpp", "api.cpp", "noalloc.cu", "selftest.cu", "server.cpp",
            "producer.cu"]
 HEADERS = ["common.cuh", "engine.h", "exec.h", "plan.h", "plan_impl.h",
-           "tune.h"]
+           "tune.h", "buffer_cache.h"]
 
 
 def _newer(target, deps):

@@ -24,6 +24,9 @@ const char *last_error();
                                              : LIBPT_ERR_CUDA;            \
     }                                                                     \
   } while (0)
+// Process-wide id of the current CUDA context, 0 if unknown; what the library
+// keeps between calls (buffers, streams, staging) is kept by it.
+uint64_t context_id();
 // Host allocations through the libpt_set_malloc / libpt_set_free hooks.
 void *host_alloc(size_t n);
 void host_free(void *p);

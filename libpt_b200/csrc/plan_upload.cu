@@ -9,10 +9,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <list>
 #include <string>
 #include <vector>
 
+#include "buffer_cache.h"
 #include "plan_impl.h"
 #include <condition_variable>
 #include <mutex>
@@ -22,115 +22,34 @@ namespace ptb {
 
 namespace {
 
-// Device buffers kept between solves.  A solve has 20 to 80 of them, and a
-// cudaMalloc / cudaFree pair takes 0.7 ms and more (2 MB: 0.4 + 0.3, 1 GB: 0.7 +
-// 1.0): 8 of 10 ms of a host-array solve at o = 8, v = 64.  At most KEEP_BYTES
-// (1.1 % of the device's memory) are kept, the rest given up, and all of them
-// when an allocation of the library fails.  A buffer comes back only after the
-// stream that used it has been waited for, so any thread and stream may take it
-// next.  Buffers belong to the context they were made in (its process-wide id:
-// a reset device has a new one, and nothing of the old is handed out).  A CUDA
-// memory pool was measured instead: it maps and unmaps at 5 ms per GB each way
-// whenever the buffers of two solves do not fit its free space alike (FP32 upt
-// 12/120/11/122: 58 to 200 ms a call).
-constexpr size_t KEEP_BYTES = (size_t)2 << 30;
-constexpr size_t KEEP_BUFFER = (size_t)1280 << 20;   // larger ones are not kept
-
-class BufferCache {
- public:
-  static BufferCache &get() {
-    static BufferCache *c = new BufferCache();   // outlives every plan
-    return *c;
-  }
-
-  // 0: unknown (nothing is kept)
-  static uint64_t context() {
-    typedef CUresult (*GetId)(CUcontext, unsigned long long *);
-    static GetId fn = [] {
-      void *p = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      return cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) ==
-                         cudaSuccess &&
-                     q == cudaDriverEntryPointSuccess
-                 ? reinterpret_cast<GetId>(p)
-                 : nullptr;
-    }();
-    unsigned long long id = 0;
-    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
-  }
-
-  // whole 64 KiB (2 MiB from there on), so that sizes of like solves meet
-  static size_t rounded(size_t n) {
-    const size_t g = n <= ((size_t)2 << 20) ? (size_t)64 << 10 : (size_t)2 << 20;
-    return (n + g - 1) & ~(g - 1);
-  }
-
-  // The smallest kept buffer of n bytes or little more, or null.
-  void *take(uint64_t ctx, size_t n, size_t *size) {
-    std::lock_guard<std::mutex> g(mu_);
-    auto best = kept_.end();
-    for (auto it = kept_.begin(); it != kept_.end(); ++it)
-      if (it->ctx == ctx && it->n >= n && it->n <= n + n / 4 + ((size_t)1 << 20) &&
-          (best == kept_.end() || it->n < best->n))
-        best = it;
-    if (best == kept_.end()) return nullptr;
-    void *p = best->p;
-    *size = best->n;
-    bytes_ -= best->n;
-    kept_.erase(best);
-    return p;
-  }
-
-  // Keeps a buffer nothing on the device uses any more (of the current
-  // context ctx), giving up the oldest ones beyond KEEP_BYTES.
-  void give(uint64_t ctx, void *p, size_t n) {
-    std::vector<void *> drop;
-    if (n > KEEP_BUFFER) {
-      drop.push_back(p);
-    } else {
-      std::lock_guard<std::mutex> g(mu_);
-      kept_.push_front({ctx, p, n, ++gives_});
-      bytes_ += n;
-      while (bytes_ > KEEP_BYTES) {
-        // the oldest if it has lain unused for long, else the largest: a
-        // solve that outgrows the cache then allocates few buffers anew
-        auto out = std::prev(kept_.end());
-        if (gives_ - out->at < 512)
-          for (auto it = kept_.begin(); it != kept_.end(); ++it)
-            if (it->n > out->n) out = it;
-        if (out->ctx == ctx) drop.push_back(out->p);   // else gone with it
-        bytes_ -= out->n;
-        kept_.erase(out);
-      }
-    }
-    for (void *q : drop) cudaFree(q);
-  }
-
-  void give_up_all(uint64_t ctx) {
-    std::list<Kept> all;
-    {
-      std::lock_guard<std::mutex> g(mu_);
-      all.swap(kept_);
-      bytes_ = 0;
-    }
-    for (const Kept &k : all)
-      if (k.ctx == ctx) cudaFree(k.p);
-  }
-
- private:
-  struct Kept {
-    uint64_t ctx;
-    void *p;
-    size_t n;
-    uint64_t at;   // gives_ when it was given
-  };
-  std::mutex mu_;
-  std::list<Kept> kept_;   // most recently given first
-  size_t bytes_ = 0;
-  uint64_t gives_ = 0;
-};
+BufferCache &buffer_cache() {
+  // outlives every plan
+  static BufferCache *c = new BufferCache([](void *p) { cudaFree(p); });
+  return *c;
+}
 
 }  // namespace
+
+uint64_t context_id() {
+  typedef CUresult (*GetId)(CUcontext, unsigned long long *);
+  static GetId fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) ==
+                       cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<GetId>(p)
+               : nullptr;
+  }();
+  unsigned long long id = 0;
+  if (!fn) return 0;
+  if (fn(nullptr, &id) == CUDA_SUCCESS) return id;
+  // a thread that has not used CUDA has no current context: cudaFree makes
+  // its device's primary one current
+  return cudaFree(nullptr) == cudaSuccess && fn(nullptr, &id) == CUDA_SUCCESS
+             ? id
+             : 0;
+}
 
 int dalloc(libpt_plan *p, void **ptr, size_t bytes) {
   *ptr = nullptr;
@@ -146,15 +65,15 @@ int dalloc(libpt_plan *p, void **ptr, size_t bytes) {
     p->arena_used = off + bytes;
     return LIBPT_OK;
   }
-  BufferCache &cache = BufferCache::get();
-  const uint64_t ctx = BufferCache::context();
+  BufferCache &cache = buffer_cache();
+  const uint64_t ctx = context_id();
   size_t n = BufferCache::rounded(bytes);
   if (ctx) *ptr = cache.take(ctx, n, &n);
   if (!*ptr) {
     cudaError_t e = cudaMalloc(ptr, n);
     if (e == cudaErrorMemoryAllocation && ctx) {
       cudaGetLastError();
-      cache.give_up_all(ctx);
+      cache.give_up(ctx);
       n = bytes;
       e = cudaMalloc(ptr, n);
     }
@@ -178,8 +97,8 @@ void dfree(libpt_plan *p, void *ptr) {
     // nothing still runs on it (or the context is broken, or another one is
     // current: then it is not kept)
     if (b.ctx && cudaStreamSynchronize(p->st) == cudaSuccess &&
-        b.ctx == BufferCache::context())
-      BufferCache::get().give(b.ctx, b.p, b.n);
+        b.ctx == context_id())
+      buffer_cache().give(b.ctx, b.p, b.n);
     else
       cudaFree(b.p);
     return;
