@@ -96,6 +96,15 @@ double libpt_uft_mp(size_t oa, size_t va, size_t ob, size_t vb,
 /* Text of the last error on the calling thread ("" if none). */
 const char *libpt_last_error(void);
 
+/* Device memory between calls.  The solves (host-array, *_dev and plans) keep
+ * up to 2 GiB of the device buffers they are done with, in each CUDA context,
+ * for the next ones; libpt_rpt_dev_static keeps none.  A solve, a server or a
+ * producer of this library that finds the device full takes them back first.
+ * A program whose own allocations need the memory calls this: it frees what
+ * is kept in the current context (cudaFree: it waits for the device) and may
+ * be called at any time, from any thread. */
+int libpt_release_device_memory(void);
+
 /* ---- precision modes ---------------------------------------------------- */
 
 #define LIBPT_PREC_FP64   0   /* FP64 DMMA tensor-core contractions          */
@@ -225,8 +234,9 @@ int libpt_upt_inputs_df(size_t oa, size_t va, size_t ob, size_t vb,
  * Same arguments as the reference entry points, but every tensor is a
  * device pointer on the current device and `stream` (a cudaStream_t, may be
  * NULL for the legacy default stream) orders the work.  The call returns
- * when the energy is known.  Scratch memory is allocated with cudaMalloc and
- * released before return.  The *_mp twins take float tensors. */
+ * when the energy is known.  Scratch memory is allocated with cudaMalloc; up
+ * to 2 GiB of it stay allocated for the next solve (see
+ * libpt_release_device_memory).  The *_mp twins take float tensors. */
 
 int libpt_rpt_dev(size_t oa, size_t va, const double *d_ov,
     const double *f_ov, const double *t1, const double *t2,

@@ -233,6 +233,11 @@ LIBPT_API double libpt_uft_mp(size_t oa, size_t va, size_t ob, size_t vb,
 
 LIBPT_API const char *libpt_last_error(void) { return ptb::last_error(); }
 
+LIBPT_API int libpt_release_device_memory(void) {
+  ptb::release_kept_buffers();
+  return LIBPT_OK;
+}
+
 // ---- device-pointer twins ---------------------------------------------------
 
 LIBPT_API int libpt_rpt_dev(size_t oa, size_t va, const double *d_ov,

@@ -27,6 +27,18 @@ const char *last_error();
 // Process-wide id of the current CUDA context, 0 if unknown; what the library
 // keeps between calls (buffers, streams, staging) is kept by it.
 uint64_t context_id();
+// Frees the device buffers kept between solves in the current context;
+// returns their bytes.
+size_t release_kept_buffers();
+// A device allocation (a call that returns a cudaError_t), made once more
+// without the kept buffers when it fails.
+template <typename F>
+cudaError_t alloc_device(F f) {
+  cudaError_t e = f();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return release_kept_buffers() ? f() : e;
+}
 // Host allocations through the libpt_set_malloc / libpt_set_free hooks.
 void *host_alloc(size_t n);
 void host_free(void *p);

@@ -51,6 +51,8 @@ uint64_t context_id() {
              : 0;
 }
 
+size_t release_kept_buffers() { return buffer_cache().give_up(context_id()); }
+
 int dalloc(libpt_plan *p, void **ptr, size_t bytes) {
   *ptr = nullptr;
   if (bytes == 0) bytes = 256;

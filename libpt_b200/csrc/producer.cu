@@ -224,6 +224,13 @@ int gemm_nt(cublasHandle_t h, int m, int n, int k, const double *A, int lda,
   return LIBPT_OK;
 }
 
+// n doubles, stream-ordered.
+cudaError_t scratch(double **p, int64_t n, cudaStream_t st) {
+  return ptb::alloc_device([&] {
+    return cudaMallocAsync((void **)p, (size_t)n * sizeof(double), st);
+  });
+}
+
 int produce(size_t o_, size_t v_, size_t naux_, const double *b_oo,
             const double *b_ov, const double *b_vv, const double *t2_abab,
             double *t2, double *i_oovo, double *i_oovv, double *i_ovvv,
@@ -256,7 +263,7 @@ int produce(size_t o_, size_t v_, size_t naux_, const double *b_oo,
   // OVVV, one occupied index at a time: Z[b][(a,c)] (v^3 scratch), then the
   // abab slice [a][b][c], then its packed aaaa slice
   double *z = nullptr;
-  CK(cudaMallocAsync((void **)&z, (size_t)(v * v * v) * sizeof(double), st));
+  CK(scratch(&z, v * v * v, st));
   int r = LIBPT_OK;
   double *ovvv_ab = i_ovvv + o * v * npair;
   for (int64_t i = 0; i < o && !r; ++i) {
@@ -375,7 +382,7 @@ int produce_u(const Spin &A, const Spin &B, double *i_oovo, double *i_oovv,
                                     vb * vb * vb, va * vb * vb, vb * va * va,
                                     1});
   double *scr = nullptr;
-  CK(cudaMallocAsync((void **)&scr, (size_t)need * sizeof(double), st));
+  CK(scratch(&scr, need, st));
   int r = same_spin(A, i_oovo, i_oovv, i_ovvv, scr, st, h, q);
   if (!r) r = same_spin(B, i_oovo + vo1, i_oovv + vv1, i_ovvv + v31, scr, st,
                         h, q);
@@ -400,7 +407,10 @@ int with_blas(const char *who, void *stream, F f) {
     return LIBPT_ERR_CUDA;
   }
   cublasHandle_t h = nullptr;
-  if (b.create(&h) != CUBLAS_STATUS_SUCCESS) {
+  cublasStatus_t created = b.create(&h);
+  if (created == CUBLAS_STATUS_ALLOC_FAILED && ptb::release_kept_buffers())
+    created = b.create(&h);
+  if (created != CUBLAS_STATUS_SUCCESS) {
     ptb::set_error(std::string(who) + ": cublasCreate failed");
     return LIBPT_ERR_CUDA;
   }

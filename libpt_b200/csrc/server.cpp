@@ -519,6 +519,8 @@ LIBPT_API int libpt_server_create(size_t mem_budget, int max_active,
   S->max_active = max_active > 0 ? max_active : 64;
   int r = LIBPT_OK;
   do {
+    // the pool may have what earlier solves left allocated
+    release_kept_buffers();
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
       set_error("libpt_server_create: no CUDA device");
@@ -531,7 +533,10 @@ LIBPT_API int libpt_server_create(size_t mem_budget, int max_active,
     budget = up256(std::min(budget, fr > desc + ((size_t)1 << 30)
                                         ? fr - desc - ((size_t)1 << 30)
                                         : (size_t)0));
-    if (budget == 0 || cudaMalloc((void **)&S->pool_base, budget) != cudaSuccess) {
+    auto device = [](void **p, size_t n) {   // a concurrent solve may keep more
+      return alloc_device([&] { return cudaMalloc(p, n); });
+    };
+    if (budget == 0 || device((void **)&S->pool_base, budget) != cudaSuccess) {
       set_error("libpt_server_create: cannot reserve the device pool");
       cudaGetLastError();
       r = LIBPT_ERR_NOMEM;
@@ -539,8 +544,8 @@ LIBPT_API int libpt_server_create(size_t mem_budget, int max_active,
     }
     S->pool_bytes = budget;
     S->pool.init(budget);
-    if (cudaMalloc((void **)&S->d_desc, desc) != cudaSuccess ||
-        cudaMalloc((void **)&S->d_err, sizeof(unsigned)) != cudaSuccess ||
+    if (device((void **)&S->d_desc, desc) != cudaSuccess ||
+        device((void **)&S->d_err, sizeof(unsigned)) != cudaSuccess ||
         cudaHostAlloc((void **)&S->h_err, sizeof(unsigned),
                       cudaHostAllocDefault) != cudaSuccess) {
       set_error("libpt_server_create: allocation failed");

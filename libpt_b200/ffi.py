@@ -107,6 +107,8 @@ def lib():
     L.libpt_rpt_inputs_df.argtypes = [sz, sz, sz] + [vp] * 8 + [vp]
     L.libpt_upt_inputs_df.restype = ctypes.c_int
     L.libpt_upt_inputs_df.argtypes = [sz] * 5 + [vp] * 9 + [vp]
+    L.libpt_release_device_memory.restype = ctypes.c_int
+    L.libpt_release_device_memory.argtypes = []
     L.libpt_selftest_recip.restype = ctypes.c_int
     L.libpt_selftest_recip.argtypes = [ctypes.c_int, ctypes.c_int,
                                        ctypes.c_int, dp]
@@ -273,6 +275,12 @@ def upt_inputs_df(fa, fb, stream=None):
         out["i_ovvv"].data_ptr(), stream or 0))
     torch.cuda.synchronize()   # the inputs (and any copies above) stay alive
     return out
+
+
+def release_device_memory():
+    """Frees the device buffers kept between solves in the current context
+    (libpt_release_device_memory)."""
+    check(lib().libpt_release_device_memory())
 
 
 def selftest_recip(lo_exp, hi_exp, n):
