@@ -9,6 +9,16 @@
 
 namespace ptb {
 
+// Raises a kernel's limit of dynamic shared memory where it needs more than
+// the default 48 KiB.  The limit belongs to the current context (a second GPU
+// or a reset device starts from the default), so every launch sets it.
+template <typename K>
+cudaError_t set_smem(K kern, size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)bytes);
+}
+
 // Device-side error word (one per launch, in global memory): bit 0 = a
 // bounded wait ran out.  The host reads it after the launch and reports
 // LIBPT_ERR_TIMEOUT; the kernel itself returns instead of hanging.

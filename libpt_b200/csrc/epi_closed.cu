@@ -288,9 +288,7 @@ cudaError_t launch(const EpiItem *d_items, int grid, int nitems,
   constexpr size_t smem =
       ((FT ? 2 : 1) * (PAIR ? 3 : 6) * PB + (HASF ? 36 : 18) * GB) *
       sizeof(double);
-  const cudaError_t e = cudaFuncSetAttribute(
-      epi_closed_kernel<FT, HASF, PAIR>,
-      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = set_smem(epi_closed_kernel<FT, HASF, PAIR>, smem);
   if (e != cudaSuccess) return e;
   epi_closed_kernel<FT, HASF, PAIR>
       <<<dim3(grid, nitems), GEPI_THREADS, smem, st>>>(d_items);

@@ -582,13 +582,6 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename K>
-cudaError_t set_smem(K kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)bytes);
-}
-
-template <typename K>
 cudaError_t launch_epi(K kern, const EpiList *d_list, const EpiItem *d_items,
                        size_t smem, dim3 grid, cudaStream_t st) {
   cudaError_t e = set_smem(kern, smem);

@@ -389,9 +389,7 @@ cudaError_t launch_grp(const GemmJob *d_jobs, GemmList *d_list, int njobs,
                        int ntiles, const LaunchMaps *pm, int grid,
                        unsigned *d_err, cudaStream_t st) {
   const size_t smem = gemm_smem_bytes(BM);
-  const cudaError_t e = cudaFuncSetAttribute(
-      gemm_dmma_grp_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)smem);
+  const cudaError_t e = set_smem(gemm_dmma_grp_kernel<BM>, smem);
   if (e != cudaSuccess) return e;
   gemm_dmma_grp_kernel<BM><<<grid, Dmma<BM>::THREADS, smem, st>>>(
       *pm, d_jobs, njobs, ntiles, d_list, d_err);
@@ -402,19 +400,10 @@ template <int BM>
 cudaError_t launch(const GemmJob *d_jobs, GemmList *d_list, int njobs,
                    int ntiles, const LaunchMaps *pm, int grid, unsigned *d_err,
                    cudaStream_t st) {
-  static bool configured = false;
   const size_t smem = gemm_smem_bytes(BM);
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(
-        gemm_dmma_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(gemm_dmma_kernel_dm<BM>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  const cudaError_t e = pm ? set_smem(gemm_dmma_kernel<BM>, smem)
+                           : set_smem(gemm_dmma_kernel_dm<BM>, smem);
+  if (e != cudaSuccess) return e;
   if (pm)
     gemm_dmma_kernel<BM><<<grid, Dmma<BM>::THREADS, smem, st>>>(*pm, d_jobs, njobs,
                                                            ntiles, d_list,

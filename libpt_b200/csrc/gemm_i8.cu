@@ -518,28 +518,14 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                             err);
 }
 
-template <typename K1, typename K2>
-cudaError_t configure(K1 k1, K2 k2, int smem, bool &done) {
-  if (done) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(
-      k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-  if (e == cudaSuccess) done = true;
-  return e;
-}
-
 template <int S, int BN>
 cudaError_t launch(const GemmJob *d_jobs, GemmList *d_list, int njobs,
                    int ntiles, const LaunchMaps *pm, int grid, unsigned *d_err,
                    cudaStream_t st) {
   using C = I8Cfg<S, BN>;
-  static bool configured = false;
-  if (cudaError_t e = configure(gemm_i8_kernel<S, BN>,
-                                gemm_i8_kernel_dm<S, BN>, C::SMEM,
-                                configured))
-    return e;
+  const cudaError_t e = pm ? set_smem(gemm_i8_kernel<S, BN>, C::SMEM)
+                           : set_smem(gemm_i8_kernel_dm<S, BN>, C::SMEM);
+  if (e != cudaSuccess) return e;
   if (pm)
     gemm_i8_kernel<S, BN><<<grid, I8_THREADS, C::SMEM, st>>>(
         *pm, d_jobs, njobs, ntiles, d_list, d_err);

@@ -318,18 +318,10 @@ cudaError_t launch(const GemmJob *d_jobs, const GemmList *d_list, int njobs,
                    int ntiles, const LaunchMaps *pm, int grid,
                    const TcProducts &prods, unsigned *d_err, cudaStream_t st) {
   using C = TcCfg<KIND, BN, NPL, NACC, ST, SW, NBUF>;
-  static bool configured = false;
   auto kp = gemm_tc_kernel<KIND, BN, NPL, NACC, ST, SW, NBUF>;
   auto kd = gemm_tc_kernel_dm<KIND, BN, NPL, NACC, ST, SW, NBUF>;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(
-        kp, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               C::SMEM);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  const cudaError_t e = pm ? set_smem(kp, C::SMEM) : set_smem(kd, C::SMEM);
+  if (e != cudaSuccess) return e;
   if (pm)
     kp<<<grid, 192, C::SMEM, st>>>(*pm, d_jobs, njobs, ntiles, prods, d_err);
   else
