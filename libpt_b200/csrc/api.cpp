@@ -47,37 +47,37 @@ int fp64_precision() {
 }
 
 // Streams of the host-pointer solves, kept between calls (creating and
-// destroying one takes 0.15 to 0.8 ms): at most four idle ones a process,
-// each used by one call at a time.
+// destroying one takes 0.15 to 0.8 ms): at most four idle ones a context, each
+// used by one call at a time, and only in the context it was made in (another
+// GPU's, or a reset device's, has another id).
 struct IdleStream {
-  int dev;
+  uint64_t ctx;
   cudaStream_t st;
 };
 std::mutex g_stream_mu;
 std::vector<IdleStream> g_idle_streams;
 
-bool take_stream(cudaStream_t *st, int *dev) {
-  if (cudaGetDevice(dev) != cudaSuccess) return false;
+bool take_stream(cudaStream_t *st, uint64_t *ctx) {
+  *ctx = ptb::context_id();   // 0: unknown, nothing is kept
   {
     std::lock_guard<std::mutex> g(g_stream_mu);
     for (size_t x = 0; x < g_idle_streams.size(); ++x)
-      if (g_idle_streams[x].dev == *dev) {
+      if (g_idle_streams[x].ctx == *ctx) {
         *st = g_idle_streams[x].st;
         g_idle_streams.erase(g_idle_streams.begin() + x);
-        // a device reset since then took the stream with it
-        if (cudaStreamQuery(*st) == cudaSuccess) return true;
-        cudaGetLastError();
-        break;
+        return true;
       }
   }
   return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking) == cudaSuccess;
 }
 
-void give_stream(cudaStream_t st, int dev) {
-  {
+void give_stream(cudaStream_t st, uint64_t ctx) {
+  if (ctx) {
     std::lock_guard<std::mutex> g(g_stream_mu);
-    if (g_idle_streams.size() < 4) {
-      g_idle_streams.push_back({dev, st});
+    int idle = 0;
+    for (const IdleStream &s : g_idle_streams) idle += s.ctx == ctx;
+    if (idle < 4) {
+      g_idle_streams.push_back({ctx, st});
       return;
     }
   }
@@ -89,9 +89,9 @@ void give_stream(cudaStream_t st, int dev) {
 // (src/pt.c:208-209).
 double host_solve(const char *name, int kind, size_t oa, size_t va, size_t ob,
                   size_t vb, const void *const *args, int dtype) {
-  int dev = 0;
+  uint64_t ctx = 0;
   cudaStream_t st = nullptr;
-  if (!take_stream(&st, &dev)) {
+  if (!take_stream(&st, &ctx)) {
     ptb::set_error(cudaGetErrorString(cudaGetLastError()));
     fatal(name);
   }
@@ -114,7 +114,7 @@ double host_solve(const char *name, int kind, size_t oa, size_t va, size_t ob,
             p->prof_tune, t1 - t0, ptb::wall_seconds() - t1, p->precision,
             p->precision == LIBPT_PREC_EMU64 ? p->slices : 0);
   ptb::plan_destroy(p);
-  give_stream(st, dev);
+  give_stream(st, ctx);
   if (r) fatal(name);
   return e;
 }

@@ -51,7 +51,8 @@ int dalloc(libpt_plan *p, void **ptr, size_t bytes);
 // stream.
 void dfree(libpt_plan *p, void *ptr);
 
-// Page-locked staging for host uploads, shared by the process: two 64 MiB
+// Page-locked staging for host uploads, shared by the solves of a context (its
+// events can be recorded on that context's streams only): two 64 MiB
 // buffers used in turn, so the host copy of one chunk into page-locked
 // memory overlaps the DMA of the previous one (pageable cudaMemcpyAsync
 // copies through the driver's own small buffers, synchronously).
@@ -74,7 +75,7 @@ struct PinnedRing {
     return ok;
   }
 };
-PinnedRing &pinned_ring();
+PinnedRing &pinned_ring();   // the current context's
 // Host copy with up to 8 threads (large copies only).
 void par_memcpy(void *dst, const void *src, size_t n);
 

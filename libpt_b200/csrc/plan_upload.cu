@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -108,8 +109,11 @@ void dfree(libpt_plan *p, void *ptr) {
 }
 
 PinnedRing &pinned_ring() {
-  static PinnedRing r;
-  return r;
+  static std::mutex mu;
+  // outlives every plan
+  static auto *rings = new std::map<uint64_t, PinnedRing>();
+  std::lock_guard<std::mutex> g(mu);
+  return (*rings)[context_id()];
 }
 
 // Host copies with up to 8 threads (large chunks only): a pool of worker

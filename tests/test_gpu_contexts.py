@@ -49,6 +49,20 @@ check()
 print("ok")
 """
 
+SOLVES = """
+cases = [synth.make(k, o, v, seed=7 + v, fock=1e-3) for k, o, v in
+         (("rpt", 4, 50), ("rft", 3, 21), ("rpt", 5, 13))]
+cases.append(synth.make("upt", 4, 17, 3, 19, seed=5))
+alone = [ffi.solve_host(c) for c in cases]
+new_context()
+for ctx in (second, first, second, first):
+    use(ctx)
+    for c, e in zip(cases, alone):
+        assert ffi.solve_host(c) == e
+print("ok")
+"""
+
+
 def child(code):
     r = subprocess.run([sys.executable, "-c", HEAD.format(root=ROOT) + code],
                        capture_output=True, text=True, timeout=300)
@@ -57,3 +71,7 @@ def child(code):
 
 def test_every_contraction_kernel_launches_in_a_second_context():
     child(KERNELS)
+
+
+def test_host_solves_alternate_between_contexts():
+    child(SOLVES)
