@@ -61,6 +61,7 @@ constexpr int BN = GEMM_BN, BK = GEMM_BK, ST = GEMM_STAGES;
 // Consumer warps of a CTA: warp rows of 16 MF rows, four columns of 32.
 template <int BM>
 struct Dmma {
+  static constexpr int CTAS = BM == 48 ? 2 : 1;   // an SM
   static constexpr int WR = BM > 64 ? 2 : 1;   // warp rows
   static constexpr int MF = BM / (16 * WR);    // m16 fragments of a warp
   static constexpr int NCW = 4 * WR;
@@ -112,7 +113,9 @@ __device__ __forceinline__ void mma_stage(double (&acc)[MF][4][4],
 }
 
 // 9 or 10 warps an SM: one SM sub-partition hosts 3 of them, which bounds the
-// kernel at 168 registers per thread (16K registers per sub-partition).
+// kernel at 168 registers per thread (16K registers per sub-partition).  The
+// kernels' launch bounds ask for the CTAs an SM that dmma_grid counts on, so
+// the compiler keeps to it (158 registers, group kernels 166, no spills).
 template <int BM, bool PM, bool GRP>
 __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
                                           const GemmJob *__restrict__ jobs,
@@ -361,7 +364,7 @@ __device__ __forceinline__ void dmma_body(const LaunchMaps *pm,
 }
 
 template <int BM>
-__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, Dmma<BM>::CTAS)
     gemm_dmma_kernel(const __grid_constant__ LaunchMaps pm,
                      const GemmJob *__restrict__ jobs, int njobs, int ntiles,
                      GemmList *list, unsigned *err) {
@@ -369,7 +372,7 @@ __global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
 }
 
 template <int BM>
-__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, Dmma<BM>::CTAS)
     gemm_dmma_kernel_dm(const GemmJob *__restrict__ jobs, GemmList *list,
                         unsigned *err) {
   dmma_body<BM, false, false>(nullptr, jobs, list->njobs, list->ntiles, list, err);
@@ -377,7 +380,7 @@ __global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
 
 // Group jobs (direct launches only).
 template <int BM>
-__global__ void __launch_bounds__(Dmma<BM>::THREADS, 1)
+__global__ void __launch_bounds__(Dmma<BM>::THREADS, Dmma<BM>::CTAS)
     gemm_dmma_grp_kernel(const __grid_constant__ LaunchMaps pm,
                          const GemmJob *__restrict__ jobs, int njobs,
                          int ntiles, GemmList *list, unsigned *err) {
