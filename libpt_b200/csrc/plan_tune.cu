@@ -67,6 +67,30 @@ double probe_flops(const libpt_plan *p, int ntiles) {
   return probe;
 }
 
+// The INT8 tile variant of a width, or null.
+const I8Tile *tile_of_width(int slices, int bn) {
+  const I8Tile *tiles = nullptr;
+  const int n = i8_tiles(slices, &tiles);
+  for (int t = 0; t < n; ++t)
+    if (tiles[t].bn == bn) return &tiles[t];
+  return nullptr;
+}
+
+// A saved choice this library has the kernels for: the INT8 tile's width, or
+// the DMMA tile rows of each spin case.  Others (a tune file written by a
+// version with other variants) are measured anew.
+bool saved_choice(const libpt_plan *p, const std::string &key,
+                  std::vector<int> *choice) {
+  if (!tune_lookup(key, choice)) return false;
+  if (p->precision == LIBPT_PREC_EMU64)
+    return choice->size() == 1 && tile_of_width(p->slices, (*choice)[0]);
+  if (choice->size() != p->cases.size()) return false;
+  for (size_t ci = 0; ci < choice->size(); ++ci)
+    if (p->cases[ci].count && (*choice)[ci] != 48 && (*choice)[ci] != 96)
+      return false;
+  return true;
+}
+
 // Whether plan creation will run autotuning probes (which read operands).
 bool tune_would_probe(libpt_plan *p) {
   if (p->queue.empty() || p->precision == LIBPT_PREC_TF32X3 || g_dry)
@@ -75,7 +99,7 @@ bool tune_would_probe(libpt_plan *p) {
   const std::string key = tune_key(p->kind, p->oa, p->va, p->ob, p->vb,
                                    p->precision, emu ? p->slices : 0, p->dtype);
   std::vector<int> choice;
-  if (tune_lookup(key, &choice) || !tune_enabled()) return false;
+  if (saved_choice(p, key, &choice) || !tune_enabled()) return false;
   const I8Tile *tiles = nullptr;
   const int ntiles = emu ? i8_tiles(p->slices, &tiles) : 0;
   return probe_flops(p, ntiles) <=
@@ -90,15 +114,15 @@ int autotune(libpt_plan *p) {
   const I8Tile *tiles = nullptr;
   const int ntiles = emu ? i8_tiles(p->slices, &tiles) : 0;
   std::vector<int> choice;
-  if (tune_lookup(key, &choice)) {
-    if (emu && !choice.empty() && choice[0] >= 0 && choice[0] < ntiles) {
-      p->i8tile = tiles[choice[0]];
+  if (saved_choice(p, key, &choice)) {
+    if (emu) {
+      p->i8tile = *tile_of_width(p->slices, choice[0]);
       for (SpinCase &c : p->cases)
         if (c.count)
           if (int r = i8_encode(p, c)) return r;
-    } else if (!emu && choice.size() == p->cases.size()) {
+    } else {
       for (size_t ci = 0; ci < p->cases.size(); ++ci)
-        if (p->cases[ci].count && (choice[ci] == 48 || choice[ci] == 96))
+        if (p->cases[ci].count)
           if (int r = set_bm(p->cases[ci], choice[ci])) return r;
     }
     return upload_views(p);
@@ -159,7 +183,7 @@ int autotune(libpt_plan *p) {
       if (c.count)
         if ((r = i8_encode(p, c))) return r;
     if ((r = upload_views(p))) return r;
-    choice.assign(1, best);
+    choice.assign(1, tiles[best].bn);
   } else {
     choice.assign(p->cases.size(), 0);
     for (size_t ci = 0; ci < p->cases.size() && !r; ++ci) {
