@@ -204,6 +204,11 @@ int plan_create(int kind, size_t oa, size_t va, size_t ob, size_t vb,
                              [](double x) { return x != 0.0; });
       if (p->closed_want && (r = closed_read(p, st, p->deferred.empty() ? p->oa : 0)))
         break;
+      // the smallest groups read the OVVV rows of two occupied indices; rows
+      // still to be copied are not known yet
+      if (p->deferred.empty() &&
+          std::count(p->closed_ok.begin(), p->closed_ok.end(), 1) < 2)
+        p->closed_on = false;
     }
     if ((r = add_cases(p))) break;
     if (p->closed_want && p->closed_on && (r = closed_build(p))) {
