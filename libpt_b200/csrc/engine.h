@@ -36,8 +36,8 @@ struct GemmSeg {
     int16_t klast;      // DMMA: fours of K in the last K step (1..4); the
                         // zero columns after them are not multiplied
   };
-  int32_t a_q, a_p;     // A-view coordinates of dims 2 and 3
-  int32_t b_p;          // B-view coordinate of dim 2
+  int32_t a_q, a_p;     // A-view coordinates of dims Q and P
+  int32_t b_p;          // B-view coordinate of dim P
   int32_t ksteps;       // ceil(K_s / GEMM_BK)
 };
 
@@ -77,7 +77,7 @@ struct LaunchMaps {
 // also take the jobs array itself as a (restrict) parameter, equal to
 // list->jobs, so the compiler may keep job fields across their stores.
 // The list is also the launch's tile queue: the CTAs of the DMMA and the
-// one-CTA INT8 kernels take tiles by incrementing `next` (the reference's
+// INT8 kernels take tiles by incrementing `next` (the reference's
 // schedule(dynamic) over triples, src/pt.c:228, 353, on the device), and the
 // last CTA to finish resets `next` and `done` to zero for the next launch of
 // the same list; the host writes both as zero.

@@ -216,7 +216,11 @@ int ensure_capacity(libpt_plan *p, const std::vector<int64_t> &ents,
 int run_entries(libpt_plan *p, const std::vector<int64_t> &ents);
 
 // ---- closed-shell triples (plan_closed.cu) ----------------------------------
-// Smallest v whose restricted solves run groups.
+// Smallest v whose restricted solves run groups.  Not where they begin to pay
+// (with the padding of both forms counted they take 0.44 to 0.55 of the general
+// products from v = 24 on): solves below keep one energy, bit for bit, through
+// one-call entry points, plans, shards and the server, the contract that v >= 48
+// has only with LIBPT_CLOSED_TOL < 0.
 constexpr int CLOSED_MIN_V = 48;
 double closed_tol();
 bool closed_possible(const libpt_plan *p);
