@@ -163,7 +163,6 @@ cudaError_t gemm_tc_launch(const GemmJob *d_jobs, GemmList *d_list,
 // segment's (Q, P) coordinates are merged into a_q = a_p * Q + a_q.
 struct I8Tile {
   int bn;     // rows of C per tile (multiple of 16, S * bn <= 512)
-  int kc;     // K bytes per pipeline stage (I8_KCHUNK: two MMA K steps)
   int cost;   // relative time of a full tile's row
 };
 // Digit planes are stored in K chunks of I8_KCHUNK bytes (64: one 64-byte

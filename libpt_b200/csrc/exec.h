@@ -23,7 +23,7 @@ struct GemmGroup {
                        // 3: FP64 DMMA closed-shell groups
   int bm = 128;        // DMMA tile rows
   int slices = 0;      // INT8 digit planes
-  I8Tile tile{0, 0, 0};   // INT8 tile shape
+  I8Tile tile{0, 0};   // INT8 tile shape
   bool operator<(const GemmGroup &o) const;
   std::string name() const;
 };

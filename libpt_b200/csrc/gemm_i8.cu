@@ -535,16 +535,14 @@ cudaError_t launch(const GemmJob *d_jobs, GemmList *d_list, int njobs,
   return cudaGetLastError();
 }
 
-// The tile variants of each slice count, widest first: rows, K chunk, and the
-// time a row takes relative to the best (480 x 65536 x 480 jobs, every tile
-// full: S = 5 0.342, 0.346, 0.376 and 0.399 ms; a narrower tile moves more
-// operand bytes per product).  Every stage is one 64-byte K chunk.
-constexpr I8Tile kTiles4[] = {
-    {128, KB, 100}, {96, KB, 110}, {80, KB, 113}, {64, KB, 118}};
-constexpr I8Tile kTiles5[] = {
-    {96, KB, 100}, {80, KB, 101}, {64, KB, 103}, {48, KB, 114}};
-constexpr I8Tile kTiles6[] = {{80, KB, 107}, {64, KB, 100}, {48, KB, 110}};
-constexpr I8Tile kTiles7[] = {{64, KB, 100}};
+// The tile variants of each slice count, widest first: rows, and the time a row
+// takes relative to the best (480 x 65536 x 480 jobs, every tile full: S = 5
+// 0.342, 0.346, 0.376 and 0.399 ms; a narrower tile moves more operand bytes
+// per product).
+constexpr I8Tile kTiles4[] = {{128, 100}, {96, 110}, {80, 113}, {64, 118}};
+constexpr I8Tile kTiles5[] = {{96, 100}, {80, 101}, {64, 103}, {48, 114}};
+constexpr I8Tile kTiles6[] = {{80, 107}, {64, 100}, {48, 110}};
+constexpr I8Tile kTiles7[] = {{64, 100}};
 
 }  // namespace
 
@@ -563,7 +561,6 @@ cudaError_t gemm_i8_launch(int slices, I8Tile t, const GemmJob *d_jobs,
                            const LaunchMaps *pm, int grid, unsigned *d_err,
                            cudaStream_t st) {
   if (grid <= 0) return cudaSuccess;
-  if (t.kc != KB) return cudaErrorInvalidValue;
 #define PTB_I8(S_, BN_)                                                       \
   if (slices == S_ && t.bn == BN_)                                            \
     return launch<S_, BN_>(d_jobs, d_list, njobs, ntiles, pm, grid, d_err, st);

@@ -182,13 +182,13 @@ int plan_append(libpt_plan *p, const int64_t *ents, size_t n, PlanCursor &cur,
         gs.b_p = ijk[st.bp];
         gs.ksteps = tc ? (st.k + tc_kchunk_elems(TC_TF32) - 1) /
                              tc_kchunk_elems(TC_TF32)
-                  : i8 ? (st.k + p->i8tile.kc - 1) / p->i8tile.kc
+                  : i8 ? (st.k + I8_KCHUNK - 1) / I8_KCHUNK
                        : st.ksteps;
         if (p->precision == LIBPT_PREC_FP64)
           gs.klast = (int16_t)dmma_klast(st.k);
         else
-          gs.half_last = (int16_t)(i8 && st.k % p->i8tile.kc != 0 &&
-                                   st.k % p->i8tile.kc <= 32);
+          gs.half_last = (int16_t)(i8 && st.k % I8_KCHUNK != 0 &&
+                                   st.k % I8_KCHUNK <= 32);
       }
       jobs.push_back(g);
     }

@@ -169,9 +169,8 @@ int autotune(libpt_plan *p) {
       if (!r) r = probe_ms(p, p->cases[big], ents, &ms);
       if (!r) r = probe_ms(p, p->cases[big], ents, &ms);
       if (!r && tune_verbose())
-        std::fprintf(stderr, "libpt autotune %s: INT8 tile %dx%d, K chunk %d B: %.3f ms\n",
-                     key.c_str(), TC_BM, tiles[t].bn,
-                     tiles[t].kc, ms);
+        std::fprintf(stderr, "libpt autotune %s: INT8 tile %dx%d: %.3f ms\n",
+                     key.c_str(), TC_BM, tiles[t].bn, ms);
       if (!r && (t == 0 || ms < best_ms)) {
         best = t;
         best_ms = ms;

@@ -228,7 +228,7 @@ int kernel_case(int precision, int m, int n, int k, int reps, double *rel_err,
     job.ea = ea;
     job.eb = eb;
     job.dbits = dbits;
-    const int kc = tl.kc;
+    const int kc = I8_KCHUNK;
     for (int s2 = 0; s2 < 2; ++s2) {
       job.seg[s2].amap = 0;
       job.seg[s2].bmap = (int16_t)(1 + s2);
