@@ -43,6 +43,24 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// 8-byte asynchronous global -> shared copy; ok == false writes 0.0 (the
+// source is not read: src-size 0 zero-fills the destination).
+__device__ __forceinline__ void cp_async8(double *dst, const double *src,
+                                          bool ok) {
+  asm volatile(
+      "cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(ok ? 8 : 0)
+      : "memory");
+}
+
+// Four doubles of a contraction output (32-byte aligned; written by an
+// earlier launch).
+__device__ __forceinline__ void load4(const double *p, double *v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+      : "l"(p));
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                "r"(count));

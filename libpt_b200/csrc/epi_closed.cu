@@ -43,21 +43,6 @@ __device__ __forceinline__ void perm_blocks(int p, int &a, int &b, int &c) {
   c = (p & 1) ? lo : hi;
 }
 
-__device__ __forceinline__ void ld4(const double *p, double *v) {
-  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-               : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-               : "l"(p));
-}
-
-// 8-byte asynchronous global -> shared copy; ok == false writes 0.0.
-__device__ __forceinline__ void cp_async8(double *dst, const double *src,
-                                          bool ok) {
-  asm volatile(
-      "cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(ok ? 8 : 0)
-      : "memory");
-}
-
 // out[8] = A1[a][b][c] + A2[b][a][c] + A3[c][b][a] for a = a0 .. a0+7; a pair
 // also adds A2[b][c][a] (its A3 is A1).  b and c are inside the space, rows
 // past it are read at its last row and never used.  ldr = v pad4(v), v4 =
@@ -78,13 +63,13 @@ __device__ __forceinline__ void gather(const double *A1, const double *A2,
     x[a] = __ldg(p1 + ac * ldr);
     y[a] = __ldg(p2 + ac * v4);
   }
-  ld4(p3, z);
-  ld4(p3 + hi, z + 4);
+  load4(p3, z);
+  load4(p3 + hi, z + 4);
 #pragma unroll
   for (int a = 0; a < T; ++a) out[a] = x[a] + y[a] + z[a];
   if (PAIR) {
-    ld4(p4, z);
-    ld4(p4 + hi, z + 4);
+    load4(p4, z);
+    load4(p4 + hi, z + 4);
 #pragma unroll
     for (int a = 0; a < T; ++a) out[a] += z[a];
   }

@@ -83,14 +83,6 @@ __device__ double block_sum(double x) {
 
 // ---------------------------------------------------------------- aaa ----
 
-// Four doubles of a contraction output (32-byte aligned; written by an
-// earlier launch).
-__device__ __forceinline__ void load4(const double *p, double *v) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-      : "l"(p));
-}
-
 // v[k] += row[p0 + k], k < 8, by aligned loads of four: p0 % 4 is the same
 // for the whole warp.  Loads past the row (ld, a multiple of 4) are moved
 // back into it; their elements are not needed.
@@ -128,16 +120,6 @@ __device__ __forceinline__ void load8(const double *row, int x0, int ld,
                                       double (&v)[8]) {
   load4(row + x0, v);
   load4(row + (x0 + 4 < ld ? x0 + 4 : x0), v + 4);
-}
-
-// 8-byte asynchronous global -> shared copy; ok == false writes 0.0 (the
-// source is not read: src-size 0 zero-fills the destination).
-__device__ __forceinline__ void cp_async8(double *dst, const double *src,
-                                          bool ok) {
-  asm volatile(
-      "cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(ok ? 8 : 0)
-      : "memory");
 }
 
 // The same for 16 bytes (both addresses 16-byte aligned).
