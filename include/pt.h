@@ -158,8 +158,8 @@ int libpt_release_device_memory(void);
  * writes max|C - C_ref| / max(|A| (|B1| + |B2|)) to *rel_err (the error over
  * the scale that bounds a dot product's rounding).  precision selects the
  * kernel (LIBPT_PREC_*, with the slice count in bits 8-14 for
- * LIBPT_PREC_EMU64, and bit 15 set for 8-bit digit planes -- a signed top
- * digit, unsigned lower digits; S <= 6 -- instead of 7-bit signed digits)
+ * LIBPT_PREC_EMU64, and bit 15 set for 8-bit balanced digit planes
+ * (S <= 6) instead of 7-bit ones)
  * and bits 16-23 a tile variant: FP64 0 = 96-row,
  * 1 = 48-row tiles; emulated FP64 the index of one of the slice count's
  * INT8 tile shapes (0 = widest); libpt_selftest_variants() counts them.
